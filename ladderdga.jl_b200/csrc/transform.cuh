@@ -6,12 +6,14 @@
 //     S(f)(q) = sum_{R in full grid} f(R) exp(-2 pi i q.R/N) = sum_{R in [0,N/2]^d} prod_a T[q_a][R_a] f(R),
 // and S(f) is again such a function, so only wedge inputs and wedge outputs are needed.  The sum is
 // evaluated axis by axis (x, then y, then z), keeping after each stage only the index ranges later
-// stages read: per vector 3D costs ~ M^4 + M^4 + Nq*M multiply-adds (M = N/2+1) instead of the
-// full-grid FFT's N^3 log N, and no data ever leaves shared memory between stages.
+// stages read (M = N/2+1 rows of (M+1)M/2 columns, M of M^2 with qy <= qx, then qz <= qy), and no data
+// ever leaves shared memory between stages.
 //
 // The convolution theorem used by the reference's conv_fft! / conv_tmp_add! then reads
 //     (1/N_k) sum_k A(k) B(k+q) = S(S(A) S(B))(q) / N_k^2.
 #pragma once
+
+#include <type_traits>
 
 #include "ldga_internal.cuh"
 
@@ -34,128 +36,259 @@ struct TransformSmem {
     static constexpr int BUF_B = DIM == 2 ? M * M : M * P2;                     // stage-1
 };
 
-// Dot product of one row of T (compile-time row/offsets when fully unrolled) with v.
-template <int M>
-__device__ __forceinline__ double2 trow(const TMat<M>& T, int row, const double2 (&v)[M]) {
-    double re = 0.0, im = 0.0;
-#pragma unroll
-    for (int a = 0; a < M; ++a) {
-        const double t = T.t[row * M + a];
-        re = fma(t, v[a].x, re);
-        im = fma(t, v[a].y, im);
-    }
-    return make_double2(re, im);
-}
-
-// Output rows of a stage are split into RS chunks so that each stage has enough independent work
-// items for the CTA (a stage has only M, P2 or M^2 columns per vector).  A chunk is a compile-time
-// row range, so every T coefficient stays an immediate constant-bank operand of its FMA; the items of
-// one chunk are padded to whole warps, so every warp applies one chunk.
-template <int DIM, int M>
-struct RowSplit {
-    static constexpr int RS = M >= 17 ? (DIM == 2 ? 4 : 2) : (M >= 9 ? 2 : 1);
-    static constexpr int CH = (M + RS - 1) / RS;
+// ------------------------------------------------------------------------------------------------
+// CUDA-core form.  One work item is one REAL column of a stage (the transform is real, so the real
+// and imaginary parts are independent): a thread reads the column's M values once, folds them, and
+// forms every row the later stages need.  The parts of a complex column sit in adjacent lanes, which
+// keeps the accesses of the interleaved (re, im) layout contiguous.
+//
+// The fold.  A column e_0 .. e_{n/2} of period n (n even) with the rows
+//     row(q) = e_0 + sum_{0<m<n/2} 2 cos(2 pi q m / n) e_m + cos(pi q) e_{n/2}
+// splits by cos(2 pi q (n/2 - m) / n) = (-1)^q cos(2 pi q m / n):
+//     odd q:   f_0 + sum_{0<m<n/4} 2 cos(2 pi q m / n) f_m,  f_m = e_m - e_{n/2-m},
+//     even q:  row q/2 of the column e'_m = e_m + e_{n/2-m} of period n/2 (e'_{n/4} = 2 e_{n/4}),
+// and so on until the period is odd.  All levels' f and the last column are M values again.  For
+// N = 32 the 17 rows take 70 multiply-adds and 31 additions instead of 289, for N = 64 309 and 63 instead of 1089, and the
+// cosines are N/4 - 1 constants, which stay in registers: with the 17 x 17 matrix as an operand every
+// FP64 instruction needed its own constant load.
+//
+// What bounds it: shared-memory column reads and writes (260 KB per 3D 32^3 vector), then the
+// barriers and loads of a CTA, which the other CTAs of its SM overlap.
+// Within a stage the items are ordered by the number of rows they need (stage y: qx, stage z: qy),
+// so a warp's lanes agree on their row loop; a second round over the items runs backwards, so a thread
+// that had few rows first has many then.
+// ------------------------------------------------------------------------------------------------
+template <int N>
+struct CosTab {
+    static constexpr int NC = N % 2 ? N / 2 + 1 : N / 4 + 1;
+    double c[NC];        // 2 cos(2 pi j / N)
 };
 
-// rows r = C CH .. C CH + CH - 1 (r < M, r <= lim) of T v, each handed to f(r, value)
-template <int M, int CH, int C, class F>
-__device__ __forceinline__ void rows_chunk(const TMat<M>& T, const double2 (&v)[M], int lim, F&& f) {
+// the levels of the fold: level l < K holds the f of period N >> l, level K the last column
+template <int N>
+struct FoldPlan {
+    static constexpr int levels() {
+        int k = 0;
+        while ((N >> k) % 2 == 0) ++k;
+        return k;
+    }
+    static constexpr int K = levels();
+    static constexpr int len(int l) {
+        const int n = N >> l;
+        return l == K ? n / 2 + 1 : ((n / 2) % 2 == 0 ? n / 4 : (n / 2 + 1) / 2);
+    }
+    static constexpr int off(int l) {
+        int o = 0;
+        for (int i = 0; i < l; ++i) o += len(i);
+        return o;
+    }
+    static constexpr int level(int q) {      // of row q
+        for (int l = 0; l < K; ++l)
+            if ((q >> l) & 1) return l;
+        return K;
+    }
+    // 2 cos(2 pi j / N) = sgn(j) c[idx(j)]
+    static constexpr int fold_j(int j) { return j % N < N - j % N ? j % N : N - j % N; }
+    static constexpr int idx(int j) { return N % 2 == 0 && 4 * fold_j(j) > N ? N / 2 - fold_j(j) : fold_j(j); }
+    static constexpr bool neg(int j) { return N % 2 == 0 && 4 * fold_j(j) > N; }
+};
+
+template <int N, int L, int ME, int M>
+__device__ __forceinline__ void fold_column(const double (&e)[ME], double (&x)[M]) {
+    using F = FoldPlan<N>;
+    constexpr int n = N >> L, o = F::off(L);
+    if constexpr (L == F::K) {
 #pragma unroll
-    for (int qq = 0; qq < CH; ++qq) {
-        const int r = C * CH + qq;
-        if (r < M && r <= lim) f(r, trow<M>(T, r, v));
+        for (int m = 0; m < F::len(L); ++m) x[o + m] = e[m];
+    } else {
+        constexpr int h = n / 2;
+#pragma unroll
+        for (int m = 0; m < F::len(L); ++m) x[o + m] = e[m] - e[h - m];
+        double s[h / 2 + 1];
+#pragma unroll
+        for (int m = 0; m <= h / 2; ++m) s[m] = e[m] + e[h - m];
+        fold_column<N, L + 1>(s, x);
     }
 }
 
-template <int DIM, int M, class F>
-__device__ __forceinline__ void rows_of(int chunk, const TMat<M>& T, const double2 (&v)[M], int lim, F&& f) {
-    using R = RowSplit<DIM, M>;
-    if (chunk == 0) rows_chunk<M, R::CH, 0>(T, v, lim, f);
-    if constexpr (R::RS > 1) { if (chunk == 1) rows_chunk<M, R::CH, 1>(T, v, lim, f); }
-    if constexpr (R::RS > 2) { if (chunk == 2) rows_chunk<M, R::CH, 2>(T, v, lim, f); }
-    if constexpr (R::RS > 3) { if (chunk == 3) rows_chunk<M, R::CH, 3>(T, v, lim, f); }
-}
-
-// for it in [0, RS * IPC): chunk = it / IPC, local item = it % IPC (< n), IPC = n rounded up to 32
-template <int DIM, int M, class Body>
-__device__ __forceinline__ void for_items(int n, Body&& body) {
-    using R = RowSplit<DIM, M>;
-    const int ipc = (n + 31) & ~31;
-    for (int it = threadIdx.x; it < R::RS * ipc; it += blockDim.x) {
-        const int chunk = it / ipc, loc = it - chunk * ipc;
-        if (loc < n) body(chunk, loc);
+// body(std::integral_constant<int, i>) for i = A .. B - 1
+template <int A, int B, class Body>
+__device__ __forceinline__ void static_for(Body&& body) {
+    if constexpr (A < B) {
+        body(std::integral_constant<int, A>{});
+        static_for<A + 1, B>(body);
     }
 }
 
-// Apply S to `np` vectors: in[p*NQ + q] (wedge-indexed).  `consume(p, q_wedge, value)` receives
-// every output exactly once.  bufA holds the inputs and is overwritten (3D stage 2); bufB is scratch.
-// All threads of the CTA must call this; it synchronises internally and on exit.
-template <int DIM, int M, class Consumer>
-__device__ void sym_transform(int np, double2* bufA, double2* bufB, const TMat<M>& T, Consumer&& consume) {
+// rows r <= lim of the folded column, CH at a time, each in increasing m
+template <int N, int CH, int R0 = 0, int M, class F>
+__device__ __forceinline__ void rows_real(const double (&c)[CosTab<N>::NC], const double (&x)[M], int lim, F&& f) {
+    using P = FoldPlan<N>;
+    if constexpr (R0 < M) {
+        if (R0 > lim) return;
+        constexpr int R1 = R0 + CH < M ? R0 + CH : M;
+        double acc[CH];
+        static_for<R0, R1>([&](auto qc) {
+            constexpr int q = decltype(qc)::value, l = P::level(q), o = P::off(l);
+            double y = x[o];
+            static_for<1, P::len(l)>([&](auto mc) {
+                constexpr int m = decltype(mc)::value, j = P::idx(q * m);
+                y = fma(P::neg(q * m) ? -c[j] : c[j], x[o + m], y);
+            });
+            acc[q - R0] = y;
+        });
+#pragma unroll
+        for (int i = 0; i < R1 - R0; ++i)
+            if (R0 + i <= lim) f(R0 + i, acc[i]);
+        rows_real<N, CH, R0 + CH>(c, x, lim, f);
+    }
+}
+
+template <int DIM, int N>
+struct TransformPlan {
+    static constexpr int M = N / 2 + 1;
     using S = TransformSmem<DIM, M>;
-    constexpr int P2 = S::P2;
-    constexpr int NQ = S::NQ;
+    static constexpr int COLS = DIM == 2 ? M : S::P2;             // complex columns of stages x and (3D) z
+    // vectors per CTA at once: the count that fills whole warps best within 320 threads
+    static constexpr int pick() {
+        int best = 1;
+        double beff = 0.0;
+        for (int np = 1; np <= 16; ++np) {
+            const int items = np * 2 * COLS, nt = (items + 31) / 32 * 32;
+            if (np > 1 && (nt > 320 || (size_t)np * (S::BUF_A + S::BUF_B) * 16 > 112 * 1024)) break;
+            double eff = (double)items / nt;
+            if (nt < 96) eff *= 0.5;
+            if (eff > beff + 0.02) { beff = eff; best = np; }
+        }
+        return best;
+    }
+    static constexpr int NP = pick();
+    // threads: an item of stages x each, and at most 3 (3D) or 4 (2D) wedge points of the loads and stores
+    static constexpr int LDQ = DIM == 3 ? 3 : 4;
+    static constexpr int NT_I = (NP * 2 * COLS + 31) / 32 * 32, NT_L = ((NP * S::NQ + LDQ - 1) / LDQ + 31) / 32 * 32;
+    static constexpr int NT = NT_L > NT_I && NT_L <= 352 ? NT_L : NT_I;
+    // one vector per CTA on its own SM (the EoM inverse): threads for stage y (3D) or the loads (2D)
+    static constexpr int NT_ONE_W = (DIM == 3 ? 2 * M * M + 31 : (S::NQ + 1) / 2 + 31) / 32 * 32;
+    static constexpr int NT_ONE = NT_ONE_W > 640 ? 640 : (NT_ONE_W > NT ? NT_ONE_W : NT);
+    static constexpr size_t SMEM1 = (size_t)(S::BUF_A + S::BUF_B) * sizeof(double2);
+    // resident CTAs the register allocation must allow: a column takes 2 M registers, its cosines N/2
+    static constexpr int THREADS_SM = DIM == 3 ? 704 : 640;
+    static constexpr int minb() {
+        int b = THREADS_SM / NT;
+        const int bs = (int)((size_t)224 * 1024 / (NP * SMEM1 + 1024));
+        if (b > bs) b = bs;
+        if (b > 16) b = 16;
+        return b < 1 ? 1 : b;
+    }
+    static constexpr int MINB = minb();
+    // rows formed together: in stage x every row is needed; in the others only rows <= a column's limit
+    static constexpr int CHX = (M + (M + 6) / 7 - 1) / ((M + 6) / 7);
+    static constexpr int CHY = (M + (M + 3) / 4 - 1) / ((M + 3) / 4);
+};
+
+// body(item) for item in [0, n): round 0 forwards, round 1 backwards, ...
+template <class Body>
+__device__ __forceinline__ void for_items_folded(int n, Body&& body) {
+    const int nt = blockDim.x;
+#pragma unroll 1
+    for (int k = 0, lo = 0; lo < n; ++k, lo += nt) {
+        const int hi = min(lo + nt, n);
+        const int it = (k & 1) ? hi - 1 - (int)threadIdx.x : lo + (int)threadIdx.x;
+        if (it >= lo && it < hi) body(it);
+    }
+}
+
+__host__ __device__ __forceinline__ constexpr int tri(int a) { return a * (a + 1) / 2; }
+__host__ __device__ __forceinline__ constexpr int tet(int a) { return a * (a + 1) * (a + 2) / 6; }
+
+// Apply S to `np` vectors held in bufA as [p][NQ] (wedge-indexed); returns the buffer (bufA in 2D,
+// bufB in 3D) that then holds the result in the same layout.  Both buffers are overwritten.  All
+// threads of the CTA must call this after a barrier behind their writes of bufA; it ends on a barrier.
+template <int DIM, int N>
+__device__ double2* sym_transform(int np, double2* bufA, double2* bufB, const CosTab<N>& T) {
+    using P = TransformPlan<DIM, N>;
+    using S = typename P::S;
+    constexpr int M = P::M, P2 = S::P2, NQ = S::NQ;
+    double* A = reinterpret_cast<double*>(bufA);
+    double* B = reinterpret_cast<double*>(bufB);
+    double c[CosTab<N>::NC];
+#pragma unroll
+    for (int j = 0; j < CosTab<N>::NC; ++j) {
+        c[j] = T.c[j];
+        asm volatile("" : "+d"(c[j]));   // a register from here on, not a constant reloaded at each use
+    }
     if constexpr (DIM == 2) {
         // stage x: W1[qx][b] = sum_a T[qx][a] f(a, b)
-        for_items<DIM, M>(np * M, [&](int chunk, int it) {
-            const int p = it / M, b = it - p * M;
-            double2 v[M];
+        for_items_folded(np * M * 2, [&](int it) {
+            const int part = it & 1, r = it >> 1, p = r / M, b = r - p * M;
+            const double* in = A + 2 * p * NQ + part;
+            const int tb = tri(b);
+            double v[M], x[M];
 #pragma unroll
-            for (int a = 0; a < M; ++a) v[a] = bufA[p * NQ + sidx2(a, b)];
-            double2* w = bufB + p * (M * M);
-            rows_of<DIM, M>(chunk, T, v, M - 1, [&](int qx, double2 y) { w[qx * M + b] = y; });
+            for (int a = 0; a < M; ++a) v[a] = in[2 * (a <= b ? tb + a : tri(a) + b)];
+            fold_column<N, 0>(v, x);
+            double* w = B + 2 * (p * (M * M) + b) + part;
+            rows_real<N, P::CHX>(c, x, M - 1, [&](int qx, double y) { w[2 * qx * M] = y; });
         });
         __syncthreads();
-        // stage y: out(qx, qy) = sum_b T[qy][b] W1[qx][b], qy <= qx
-        for_items<DIM, M>(np * M, [&](int chunk, int it) {
-            const int p = it / M, qx = it - p * M;
-            if (chunk * RowSplit<DIM, M>::CH > qx) return;
-            double2 v[M];
-            const double2* w = bufB + p * (M * M) + qx * M;
+        // stage y: out(qx, qy) = sum_b T[qy][b] W1[qx][b], qy <= qx; columns in order of qx
+        for_items_folded(np * M * 2, [&](int it) {
+            const int part = it & 1, r = it >> 1, qx = r / np, p = r - qx * np;
+            const double* w = B + 2 * (p * (M * M) + qx * M) + part;
+            double v[M], x[M];
 #pragma unroll
-            for (int b = 0; b < M; ++b) v[b] = w[b];
-            rows_of<DIM, M>(chunk, T, v, qx, [&](int qy, double2 y) { consume(p, widx2(qx, qy), y); });
+            for (int b = 0; b < M; ++b) v[b] = w[2 * b];
+            fold_column<N, 0>(v, x);
+            double* o = A + 2 * (p * NQ + tri(qx)) + part;
+            rows_real<N, P::CHY>(c, x, qx, [&](int qy, double y) { o[2 * qy] = y; });
         });
         __syncthreads();
+        return bufA;
     } else {
         // stage x: W1[qx][(b,c)] = sum_a T[qx][a] f(a, b, c) for b >= c
-        for_items<DIM, M>(np * P2, [&](int chunk, int it) {
-            const int p = it / P2, j = it - p * P2;
-            int b, c;
-            decode_pair(j, b, c);
-            double2 v[M];
+        for_items_folded(np * P2 * 2, [&](int it) {
+            const int part = it & 1, r = it >> 1, p = r / P2, j = r - p * P2;
+            int b, cc;
+            decode_pair(j, b, cc);
+            const double* in = A + 2 * p * NQ + part;
+            const int i0 = tet(b) + tri(cc), i1 = tet(b) + cc, i2 = tri(b) + cc;   // a <= c, c < a <= b, a > b
+            double v[M], x[M];
 #pragma unroll
-            for (int a = 0; a < M; ++a) v[a] = bufA[p * NQ + sidx3(a, b, c)];
-            double2* w = bufB + p * (M * P2);
-            rows_of<DIM, M>(chunk, T, v, M - 1, [&](int qx, double2 y) { w[qx * P2 + j] = y; });
+            for (int a = 0; a < M; ++a) v[a] = in[2 * (a <= cc ? i0 + a : a <= b ? i1 + tri(a) : i2 + tet(a))];
+            fold_column<N, 0>(v, x);
+            double* w = B + 2 * (p * (M * P2) + j) + part;
+            rows_real<N, P::CHX>(c, x, M - 1, [&](int qx, double y) { w[2 * qx * P2] = y; });
         });
         __syncthreads();
-        // stage y: W2[(qx,qy)][c] = sum_b T[qy][b] W1[qx][(b,c)], qy <= qx  (W1 symmetric in b,c)
-        for_items<DIM, M>(np * M * M, [&](int chunk, int it) {
-            const int p = it / (M * M), r = it - p * (M * M);
-            const int qx = r / M, c = r - qx * M;
-            if (chunk * RowSplit<DIM, M>::CH > qx) return;
-            double2 v[M];
-            const double2* w = bufB + p * (M * P2) + qx * P2;
+        // stage y: W2[(qx,qy)][c] = sum_b T[qy][b] W1[qx][(b,c)], qy <= qx (W1 symmetric in b, c)
+        for_items_folded(np * M * M * 2, [&](int it) {
+            const int part = it & 1, r = it >> 1, qx = r / (np * M), s = r - qx * (np * M), p = s / M, cc = s - p * M;
+            const double* w = B + 2 * (p * (M * P2) + qx * P2) + part;
+            const int tc = tri(cc);
+            double v[M], x[M];
 #pragma unroll
-            for (int b = 0; b < M; ++b) v[b] = w[sidx2(b, c)];
-            double2* o = bufA + p * S::BUF_A;
-            rows_of<DIM, M>(chunk, T, v, qx, [&](int qy, double2 y) { o[widx2(qx, qy) * M + c] = y; });
+            for (int b = 0; b < M; ++b) v[b] = w[2 * (b <= cc ? tc + b : tri(b) + cc)];
+            fold_column<N, 0>(v, x);
+            double* o = A + 2 * (p * S::BUF_A + tri(qx) * M + cc) + part;
+            rows_real<N, P::CHY>(c, x, qx, [&](int qy, double y) { o[2 * qy * M] = y; });
         });
         __syncthreads();
-        // stage z: out(qx,qy,qz) = sum_c T[qz][c] W2[(qx,qy)][c], qz <= qy
-        for_items<DIM, M>(np * P2, [&](int chunk, int it) {
-            const int p = it / P2, pq = it - p * P2;
-            int qx, qy;
-            decode_pair(pq, qx, qy);
-            if (chunk * RowSplit<DIM, M>::CH > qy) return;
-            double2 v[M];
-            const double2* w = bufA + p * S::BUF_A + pq * M;
+        // stage z: out(qx,qy,qz) = sum_c T[qz][c] W2[(qx,qy)][c], qz <= qy; columns by falling qy
+        for_items_folded(np * P2 * 2, [&](int it) {
+            const int part = it & 1, r = it >> 1, j = r / np, p = r - j * np;
+            int bb, cc;
+            decode_pair(j, bb, cc);
+            const int qy = M - 1 - bb, qx = M - 1 - cc;
+            const double* w = A + 2 * (p * S::BUF_A + (tri(qx) + qy) * M) + part;
+            double v[M], x[M];
 #pragma unroll
-            for (int c = 0; c < M; ++c) v[c] = w[c];
-            rows_of<DIM, M>(chunk, T, v, qy, [&](int qz, double2 y) { consume(p, widx3(qx, qy, qz), y); });
+            for (int m = 0; m < M; ++m) v[m] = w[2 * m];
+            fold_column<N, 0>(v, x);
+            double* o = B + 2 * (p * NQ + tet(qx) + tri(qy)) + part;
+            rows_real<N, P::CHY>(c, x, qy, [&](int qz, double y) { o[2 * qz] = y; });
         });
         __syncthreads();
+        return bufB;
     }
 }
 
@@ -240,8 +373,8 @@ __device__ __forceinline__ void tc_stage(const TFrag<M>& F, int ncol, ColB&& col
 }
 
 // sym_transform's interface and buffers on the tensor path.
-template <int DIM, int M, class Consumer>
-__device__ void sym_transform_tc(int np, double2* bufA, double2* bufB, const TMat<M>& T, Consumer&& consume) {
+template <int DIM, int M>
+__device__ double2* sym_transform_tc(int np, double2* bufA, double2* bufB, const TMat<M>& T) {
     using S = TransformSmem<DIM, M>;
     constexpr int P2 = S::P2;
     constexpr int NQ = S::NQ;
@@ -258,8 +391,9 @@ __device__ void sym_transform_tc(int np, double2* bufA, double2* bufB, const TMa
         tc_stage<M>(F, np * M,
             [&](int j, int k) { const int p = j / M, qx = j - p * M; return bufB[p * (M * M) + qx * M + k]; },
             [&](int j) { return j % M; },
-            [&](int j, int r, double2 v) { const int p = j / M, qx = j - p * M; consume(p, widx2(qx, r), v); });
+            [&](int j, int r, double2 v) { const int p = j / M, qx = j - p * M; bufA[p * NQ + widx2(qx, r)] = v; });
         __syncthreads();
+        return bufA;
     } else {
         // stage x: W1[qx][(b, c)] = sum_a T[qx][a] f(a, b, c), b >= c; column j = (p, pair)
         tc_stage<M>(F, np * P2,
@@ -296,27 +430,31 @@ __device__ void sym_transform_tc(int np, double2* bufA, double2* bufB, const TMa
                 const int p = j / P2, pq = j - p * P2;
                 int qx, qy;
                 decode_pair(pq, qx, qy);
-                consume(p, widx3(qx, qy, r), v);
+                bufB[p * NQ + widx3(qx, qy, r)] = v;
             });
         __syncthreads();
+        return bufB;
     }
 }
 
-// the CUDA-core or the tensor-path form, chosen at compile time
-template <int DIM, int M, bool TC, class Consumer>
-__device__ __forceinline__ void sym_transform_any(int np, double2* bufA, double2* bufB, const TMat<M>& T,
-                                                  Consumer&& consume) {
-    if constexpr (TC) sym_transform_tc<DIM, M>(np, bufA, bufB, T, consume);
-    else sym_transform<DIM, M>(np, bufA, bufB, T, consume);
+// the CUDA-core or the tensor-path form, chosen at compile time, and its coefficient operand
+template <int N, bool TC>
+using TransformCoef = std::conditional_t<TC, TMat<N / 2 + 1>, CosTab<N>>;
+
+template <int DIM, int N, bool TC>
+__device__ __forceinline__ double2* sym_transform_any(int np, double2* bufA, double2* bufB,
+                                                      const TransformCoef<N, TC>& T) {
+    if constexpr (TC) return sym_transform_tc<DIM, N / 2 + 1>(np, bufA, bufB, T);
+    else return sym_transform<DIM, N>(np, bufA, bufB, T);
 }
 
 }  // namespace ldga
 
-// Instantiation list: (DIM, M) pairs the library is built for.  M = N/2 + 1.
-//   N = 1 (one-point grid of the local quantities) in 2D and 3D
-//   2D: N = 2, 4, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64
-//   3D: N = 2, 4, 6, 8, 10, 12, 16, 20, 24, 32
-#define LDGA_FOR_EACH_GRID(X)                                                              \
-    X(2, 1) X(3, 1) X(2, 2) X(2, 3) X(2, 4) X(2, 5) X(2, 6) X(2, 7) X(2, 9) X(2, 11) X(2, 13) X(2, 17)      \
-    X(2, 21) X(2, 25) X(2, 33)                                                             \
-    X(3, 2) X(3, 3) X(3, 4) X(3, 5) X(3, 6) X(3, 7) X(3, 9) X(3, 11) X(3, 13) X(3, 17)
+// Instantiation list: the k-grid sizes N per dimension the library is built for (N = 1: the one-point
+// grid of the local quantities).
+#define LDGA_FOR_EACH_GRID(X)                                                                          \
+    X(2, 1) X(3, 1) X(2, 2) X(2, 4) X(2, 6) X(2, 8) X(2, 10) X(2, 12) X(2, 16) X(2, 20) X(2, 24) X(2, 32) \
+    X(2, 40) X(2, 48) X(2, 64) X(2, 3) X(2, 5) X(2, 7) X(2, 9) X(2, 11) X(2, 13) X(2, 17) X(2, 21)        \
+    X(2, 25) X(2, 33) X(2, 41) X(2, 49)                                                                \
+    X(3, 2) X(3, 4) X(3, 6) X(3, 8) X(3, 10) X(3, 12) X(3, 16) X(3, 20) X(3, 24) X(3, 32) X(3, 3) X(3, 5) \
+    X(3, 7) X(3, 9) X(3, 11) X(3, 13) X(3, 17) X(3, 21) X(3, 25) X(3, 33)
