@@ -24,7 +24,8 @@
 //                       y = row sums of B^-1.
 //   LDGA_PREC_FP64      FP64 elimination of [B | 1].
 //   LDGA_PREC_MIXED     per box size the fastest of: the q-shared preconditioned iteration
-//                       (k_bse_iter: an FP32 inverse per group of 32 q, FP64 residual sweeps; at
+//                       (k_bse_iter, and k_bse_group of kernels_bse_group.cu for Nν = 42 .. 64: an FP32
+//                       inverse per group of q, FP64 residual sweeps; at
 //                       Nν = 40 both products on tensor cores: FP64 mma.sync m8n8k4 for the residual,
 //                       TF32 m16n8k8 for the correction), an FP32 elimination with FP64
 //                       iterative refinement (r = 1 - B y in FP64, the correction from the stored
@@ -32,12 +33,13 @@
 // No pivoting is done in the fast path.  Every solution is verified by its FP64 backward error
 // |1 - B y|_inf / (|B|_inf |y|_inf + 1); a matrix above 1e-12 (1e-14 for the preconditioned
 // iteration), or with a non-finite y, is flagged
-// and re-solved by a partial-pivoting FP64 LU kernel, which is also the path for box sizes that
-// have no tiled instantiation.
+// and re-solved by a partial-pivoting FP64 LU kernel, which is also the path for boxes above Nν = 112 (but
+// 120); other box sizes without kernels of their own run on the next tile.
 #include <cmath>
 #include <map>
 #include <mutex>
 
+#include "bse_common.cuh"
 #include "ldga_internal.cuh"
 #include "ns_inverse.cuh"
 
@@ -95,25 +97,6 @@ __device__ __forceinline__ V shfl_v(V v, int src) {
 __device__ __forceinline__ void named_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
-
-struct BseArgs {
-    int nq, nnu, nw, qchunk;
-    double beta, U;
-    int s;                  // -1 for d, +1 for m
-    const double2* Gamma;   // [Nnu, Nnu, Nw]
-    const double2* chi0;    // [Nq, Nnu, Nw]
-    double* chi;            // [Nq, Nw]
-    double2* gam;           // [Nq, Nnu, Nw]
-    int32_t* flags;         // [Nq, Nw]
-    unsigned long long* stats = nullptr;   // [2] k_bse_iter: residual passes and warps (may be null)
-    // k_bse_iter: a flagged matrix is also appended (q + Nq w) to fail_list at atomicAdd(fail_count)
-    int32_t* fail_list = nullptr;
-    int32_t* fail_count = nullptr;
-    int max_sweeps = 40;    // k_bse_iter: residual sweeps before a q is flagged
-    // k_bse_iter<..., ADJ = true>: right-hand sides [Nq, NL, Nw] instead of ones; the conjugate of the
-    // solution goes to gam (which may be rhs itself), chi is not written
-    const double2* rhs = nullptr;
-};
 
 __device__ __forceinline__ double2 dmk(double r, double i) { return make_double2(r, i); }
 
@@ -446,6 +429,10 @@ __global__ void __launch_bounds__(TR * TC * MPC, MINB) k_bse_tile(const BseArgs 
 // lane writes y_i = (z_i - sum) / b_ii, one named barrier, and every lane adds u_ij y_j of its column
 // of block r into the partial sums of the rows above.
 // The solution is verified by its FP64 backward error exactly like k_bse_tile (flag above 1e-12).
+// PAD: a box of a.nnu < N rows on the tile of N: rows and columns beyond it are an identity block with a
+// zero right-hand side, so y stays 0 there.  Box sizes without kernels of their own run on the next tile;
+// they had the pivoted kernel (one matrix per CTA, three barriers and two divisions per step and element
+// loops with integer divisions) for every matrix: Nnu = 34, 84 q x 27 w 625 us per channel.
 template <int N, int T>
 struct LuSmem {
     static constexpr int RT = (N + T - 1) / T;
@@ -459,13 +446,15 @@ struct LuSmem {
         (2 * RW + 2 * CW + N + N + N) * sizeof(double2) + 8 * (G / 32) * sizeof(double) + 16;
 };
 
-template <int N, int T, int MPC, int MINB, bool GSM, bool LA>
+template <int N, int T, int MPC, int MINB, bool GSM, bool LA, bool PAD>
 __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a) {
     using LS = LuSmem<N, T>;
     constexpr int RT = LS::RT, NC = LS::NC, G = LS::G;
     constexpr int CT = (NC + T - 1) / T;
     constexpr int TCN = N % T, CN = N / T;                // owner lane / tile column of the rhs
     static_assert(T <= 32 && 32 % T == 0, "a row group must sit inside one warp");
+    static_assert(!PAD || GSM, "a padded box stages Gamma(w) in shared memory");
+    const int nl = PAD ? a.nnu : N;      // rows of the box
     extern __shared__ double2 sm[];
     // Gamma(w): staged in shared memory (GSM), or read through L1/L2 when N x N does not fit
     const double2* Gsm = GSM ? sm : a.Gamma + (size_t)blockIdx.y * N * N;   // Gamma[j + N*i] at i*N + j
@@ -473,7 +462,7 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a) {
     const int g = tid / G, t = tid - g * G;
     const int tr = t / T, tc = t - (t / T) * T;
     const int lane = tid & 31;
-        const int bar = g + 1;
+    const int bar = g + 1;
     char* gs = reinterpret_cast<char*>(sm + (GSM ? N * N : 0)) + g * LS::bytes;
     double2* rowbuf = reinterpret_cast<double2*>(gs);     // [2][RW]
     double2* colbuf = rowbuf + 2 * LS::RW;                // [2][CW]
@@ -486,14 +475,21 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a) {
     const int q0 = blockIdx.x * a.qchunk;
     const int q1 = min(a.nq, q0 + a.qchunk);
     if (GSM) {
-        const double2* Gw = a.Gamma + (size_t)w * N * N;
-        for (int e = tid; e < N * N; e += blockDim.x) sm[e] = Gw[e];
+        const double2* Gw = a.Gamma + (size_t)w * nl * nl;
+        for (int e = tid; e < N * N; e += blockDim.x) {
+            if constexpr (PAD) {
+                const int i = e / N, j = e - i * N;
+                sm[e] = i < nl && j < nl ? Gw[(size_t)i * nl + j] : dmk(0.0, 0.0);
+            } else {
+                sm[e] = Gw[e];
+            }
+        }
     }
     __syncthreads();
 
     for (int q = q0 + g; q < q1; q += MPC) {
-        const double2* c0p = a.chi0 + (size_t)q + (size_t)a.nq * ((size_t)N * w);
-        for (int i = t; i < N; i += G) dinv[i] = cinv(c0p[(size_t)a.nq * i]);
+        const double2* c0p = a.chi0 + (size_t)q + (size_t)a.nq * ((size_t)nl * w);
+        for (int i = t; i < N; i += G) dinv[i] = !PAD || i < nl ? cinv(c0p[(size_t)a.nq * i]) : dmk(1.0, 0.0);
         named_barrier(bar, G);
         // ---- load the tile of [B | 1], B_ij = Gamma[j, i] + delta_ij / chi0(q, i, w); the diagonal
         // i == j can only fall into tile (ra, ra) of the threads with tr == tc
@@ -510,7 +506,7 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a) {
                         v = Gsm[i * N + j];
                         if (c == ra && tr == tc) v = cadd(v, dinv[i]);
                     } else if (j == N) {
-                        v = dmk(1.0, 0.0);
+                        v = dmk(!PAD || i < nl ? 1.0 : 0.0, 0.0);
                     }
                 }
                 b[ra][c] = v;
@@ -691,7 +687,7 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a) {
                 accr.y += __shfl_xor_sync(0xffffffffu, accr.y, o);
                 rown += __shfl_xor_sync(0xffffffffu, rown, o);
             }
-            if (i < N && tc == 0) {
+            if (i < nl && tc == 0) {
                 st[0] = fmax(st[0], fabs(1.0 - accr.x) + fabs(accr.y));
                 st[1] = fmax(st[1], fabs(y[ra].x) + fabs(y[ra].y));
                 st[2] = fmax(st[2], rown);
@@ -712,8 +708,8 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a) {
 #pragma unroll
         for (int ra = 0; ra < RT; ++ra) {
             const int i = tr + T * ra;
-            if (i < N && tc == 0) {
-                const size_t ci = (size_t)q + (size_t)a.nq * (i + (size_t)N * w);
+            if (i < nl && tc == 0) {
+                const size_t ci = (size_t)q + (size_t)a.nq * (i + (size_t)nl * w);
                 a.gam[ci] = cscale(cmul(y[ra], dinv[i]), rf);
             }
         }
@@ -2723,12 +2719,12 @@ int run_tile(ldga_ctx* ctx, const BseArgs& a0) {
     return LDGA_OK;
 }
 
-template <int N, int T, int MPC, int MINB, bool GSM = true, bool LA = LDGA_LU_LOOKAHEAD>
+template <int N, int T, int MPC, int MINB, bool GSM = true, bool LA = LDGA_LU_LOOKAHEAD, bool PAD = false>
 int run_lu(ldga_ctx* ctx, const BseArgs& a0) {
     BseArgs a = a0;
     const int threads = T * T * MPC;
     const size_t sm = (GSM ? (size_t)N * N * sizeof(double2) : 0) + MPC * LuSmem<N, T>::bytes;
-    auto kern = k_bse_lu<N, T, MPC, MINB, GSM, LA>;
+    auto kern = k_bse_lu<N, T, MPC, MINB, GSM, LA, PAD>;
     LDGA_CUDA(ctx, set_smem(ctx, kern, sm));
     int chunk = 4 * MPC;
     while (chunk > MPC && (long)((a.nq + chunk - 1) / chunk) * a.nw < 8 * 148) chunk -= MPC;
@@ -2790,21 +2786,8 @@ int run_iter_impl(ldga_ctx* ctx, const BseArgs& a, const BseArgs* a_d) {
     auto kern = k_bse_iter<N, LPQ, QPL, MINB, GSM, TC, DM, P2, NS, NL, ADJ>;
     LDGA_CUDA(ctx, set_smem(ctx, kern, S::bytes));
     StageTimer st_(ctx, LDGA_STAGE_BSE);
-    // the q order depends on chi0 only: the second channel of the same bubble reuses it
-    if (ctx->qperm_gen != ctx->chi0_gen) {
-        if (a.nq <= 4096) {
-            int P = 32;
-            while (P < a.nq) P <<= 1;
-            const size_t smq = (size_t)P * (sizeof(double) + sizeof(int));
-            LDGA_CUDA(ctx, set_smem(ctx, k_bse_qorder, smq));
-            k_bse_qorder<<<a.nw, 1024, smq, ctx->stream>>>(a.nq, NL, a.chi0, ctx->d_qperm);
-            LDGA_LAUNCHED(ctx, "k_bse_qorder");
-        } else {
-            k_bse_qorder_id<<<148, 256, 0, ctx->stream>>>(a.nq, a.nw, ctx->d_qperm);
-            LDGA_LAUNCHED(ctx, "k_bse_qorder_id");
-        }
-        ctx->qperm_gen = ctx->chi0_gen;
-    }
+    const int qo = bse_ensure_qorder(ctx, a, NL);
+    if (qo != LDGA_OK) return qo;
     dim3 grid((a.nq + kIterQ - 1) / kIterQ, a.nw, a_d ? 2 : 1);
     kern<<<grid, kIterQ * LPQ / QPL, S::bytes, ctx->stream>>>(a, a_d ? *a_d : a, ctx->d_qperm);
     LDGA_LAUNCHED(ctx, "k_bse_iter");
@@ -2821,6 +2804,15 @@ template <int N, int LPQ, int MINB, int QPL = 1, bool GSM = true, bool TC = fals
           bool NS = false, int NL = N>
 int run_iter_pair(ldga_ctx* ctx, const BseArgs& a_m, const BseArgs& a_d) {
     return run_iter_impl<N, LPQ, MINB, QPL, GSM, TC, DM, P2, NS, NL>(ctx, a_m, &a_d);
+}
+
+template <int TILE>
+int run_group(ldga_ctx* ctx, const BseArgs& a) {
+    return run_bse_group(ctx, TILE, a, nullptr);
+}
+template <int TILE>
+int run_group_pair(ldga_ctx* ctx, const BseArgs& a_m, const BseArgs& a_d) {
+    return run_bse_group(ctx, TILE, a_m, &a_d);
 }
 
 struct BseVariant {
@@ -2858,6 +2850,7 @@ LDGA_ITER_BOX(16, 4, 4, 16, 4, "iter8x2dm2ns16:4")
 LDGA_ITER_BOX(20, 4, 4, 24, 4, "iter8x2dm2ns24:4")
 LDGA_ITER_BOX(30, 4, 3, 32, 3, "iter8x2dm2ns32:3")
 #undef LDGA_ITER_BOX
+constexpr int kIter30 = 3;   // the tensor-core iteration in mixed_30
 const BseVariant fp64_40[] = {{&run_lu<40, 8, 1, 6>, "lu8:6"}, {&run_lu<40, 8, 1, 4>, "lu8:4"},
                               {&run_lu<40, 8, 1, 5>, "lu8:5"}};
 // the default: the group inverse by Newton-Schulz on tcgen05 tensor cores (Gauss-Jordan as its fallback)
@@ -2876,10 +2869,8 @@ const BseVariant fp64_60[] = {{&run_lu<60, 16, 1, 2>, "lu16:2"}, {&run_lu<60, 16
                               {&run_lu<60, 16, 1, 3>, "lu16:3"}};
 // MIXED may pick any configuration whose results meet the FP64 backward-error bound, the FP64 LU
 // included: at Nν = 60 and 120 that is the fastest one measured
-// the preconditioned iteration on tiles padded to 64 (an identity block below the box), both products
-// on tensor cores and the group inverse on tcgen05, one 128-thread CTA per SM (151 KB of shared memory)
-const BseVariant mixed_60[] = {{&run_iter<64, 8, 1, 2, true, true, true, true, true, 60>, "iter8x2dm2ns64:1",
-                                &run_iter_pair<64, 8, 1, 2, true, true, true, true, true, 60>},
+// the grouped preconditioned iteration (kernels_bse_group.cu) on tiles padded to 64
+const BseVariant mixed_60[] = {{&run_group<64>, "iterg64", &run_group_pair<64>},
                                {&run_lu<60, 16, 1, 2>, "lu16:2"}, {&run_lu32<60, 16, 1, 3>, "lu32x16:3"},
                                {&run_lu32<60, 16, 1, 2>, "lu32x16:2"}, {&run_iter<60, 8, 1>, "iter"}};
 const BseVariant inv_60[] = {{&run_tile<60, 16, 16, 1, 1, double, LDGA_PREC_FP64_INV>, "gj16x1"}};
@@ -2895,6 +2886,34 @@ const BseVariant mixed_120[] = {{&run_jacobi<120, 32, 4, true>, "jac", &run_jaco
                                 {&run_jacobi<120, 16, 2, true>, "jac16:2", &run_jacobi_pair<120, 16, 2, true>},
                                 {&run_lu<120, 16, 1, 1, false>, "lu16g:1"}, {&run_lu32<120, 16, 1, 1, false>, "lu32x16g:1"}};
 
+// Box sizes without kernels of their own: the LU on the next tile up (padded), all modes; in MIXED the
+// grouped iteration above Nnu = 40, where the elimination's N^3 outgrows it.  Nnu > 112 (but 120): the
+// pivoted kernel (a 128 x 129 register tile spills, Gamma(w) outgrows shared memory).
+template <int N, int T, int MINB>
+constexpr BseVariant padded_lu(const char* name) {
+    return {&run_lu<N, T, 1, MINB, true, LDGA_LU_LOOKAHEAD, true>, name};
+}
+const BseVariant padded_lus[] = {padded_lu<8, 8, 8>("lu8p8"),     padded_lu<16, 8, 8>("lu8p16"),
+                                 padded_lu<24, 8, 8>("lu8p24"),   padded_lu<32, 8, 6>("lu8p32"),
+                                 padded_lu<40, 8, 6>("lu8p40"),   padded_lu<48, 16, 3>("lu16p48"),
+                                 padded_lu<56, 16, 2>("lu16p56"), padded_lu<64, 16, 2>("lu16p64"),
+                                 padded_lu<80, 16, 1>("lu16p80"), padded_lu<96, 16, 1>("lu16p96"),
+                                 padded_lu<112, 16, 1>("lu16p112")};
+const int padded_tiles[] = {8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 112};
+const BseVariant padded_iters[] = {{&run_group<48>, "iterg48", &run_group_pair<48>},
+                                   {&run_group<56>, "iterg56", &run_group_pair<56>},
+                                   {&run_group<64>, "iterg64", &run_group_pair<64>}};
+
+int padded_variant(int nnu, int prec, const BseVariant** out) {
+    *out = nullptr;
+    for (int i = 0; i < (int)(sizeof(padded_tiles) / sizeof(int)); ++i)
+        if (nnu <= padded_tiles[i]) {
+            *out = prec == LDGA_PREC_MIXED && i >= 5 && i <= 7 ? &padded_iters[i - 5] : &padded_lus[i];
+            return 1;
+        }
+    return 0;
+}
+
 int variants_of(int nnu, int prec, const BseVariant** out) {
 #define LDGA_BOX(N)                                                                                      \
     case N:                                                                                             \
@@ -2907,7 +2926,7 @@ int variants_of(int nnu, int prec, const BseVariant** out) {
         case 120:
             if (prec == LDGA_PREC_MIXED) { *out = mixed_120; return (int)(sizeof(mixed_120) / sizeof(BseVariant)); }
             *out = fp64_120; return (int)(sizeof(fp64_120) / sizeof(BseVariant));
-        default: *out = nullptr; return 0;
+        default: return padded_variant(nnu, prec, out);
     }
 #undef LDGA_BOX
 }
@@ -2920,6 +2939,19 @@ int tuned_index(int nnu, int prec) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find({nnu, prec});
     return it == g_tune.end() ? 0 : it->second;
+}
+
+// The configuration a launch uses: the recorded choice, else entry 0, except that at Nν = 30 grids with many
+// q take the tensor-core iteration: 2D 32^2 (153 q, Nω = 31) 256 us for both channels against the warp LU's
+// 384, 3D 16^3 (165 q) 283 against 389.  With few q the groups' diagonals spread more and matrices are
+// left to the pivoted solve, so smaller grids keep the LU.
+int chosen_variant(const ldga_ctx* ctx) {
+    const int i = tuned_index(ctx->Nnu, ctx->prec);
+    if (i == 0 && ctx->Nnu == 30 && ctx->prec == LDGA_PREC_MIXED && ctx->Nq >= 150) {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        if (g_tune.find({30, LDGA_PREC_MIXED}) == g_tune.end()) return kIter30;
+    }
+    return i;
 }
 
 // The kernels see the ω shard as a whole problem of shard_nw frequencies: every array has ω as its
@@ -3003,11 +3035,27 @@ __global__ void k_adj_chi0bar(const BseAdjArgs a) {
 
 }  // namespace
 
-bool bse_has_fast_path(int nnu) {
-    switch (nnu) {
-        case 4: case 6: case 8: case 10: case 12: case 16: case 20: case 30: case 40: case 60: case 120: return true;
-        default: return false;
+// the q order depends on chi0 only: the second channel of the same bubble reuses it
+int bse_ensure_qorder(ldga_ctx* ctx, const BseArgs& a, int nnu) {
+    if (ctx->qperm_gen == ctx->chi0_gen) return LDGA_OK;
+    if (a.nq <= 4096) {
+        int P = 32;
+        while (P < a.nq) P <<= 1;
+        const size_t smq = (size_t)P * (sizeof(double) + sizeof(int));
+        LDGA_CUDA(ctx, set_smem(ctx, k_bse_qorder, smq));
+        k_bse_qorder<<<a.nw, 1024, smq, ctx->stream>>>(a.nq, nnu, a.chi0, ctx->d_qperm);
+        LDGA_LAUNCHED(ctx, "k_bse_qorder");
+    } else {
+        k_bse_qorder_id<<<148, 256, 0, ctx->stream>>>(a.nq, a.nw, ctx->d_qperm);
+        LDGA_LAUNCHED(ctx, "k_bse_qorder_id");
     }
+    ctx->qperm_gen = ctx->chi0_gen;
+    return LDGA_OK;
+}
+
+bool bse_has_fast_path(int nnu) {
+    const BseVariant* v = nullptr;
+    return variants_of(nnu, LDGA_PREC_FP64, &v) > 0;
 }
 
 size_t bse_pivot_smem(int nnu) { return (size_t)nnu * (nnu + 1) * sizeof(double2) + 64 * sizeof(double) + 16; }
@@ -3051,7 +3099,7 @@ int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail) {
         const BseVariant* v = nullptr;
         const int nv = variants_of(ctx->Nnu, ctx->prec, &v);
         if (nv > 0) {
-            int i = tuned_index(ctx->Nnu, ctx->prec);
+            int i = chosen_variant(ctx);
             if (i >= nv) i = 0;
             st = v[i].run(ctx, a);
         } else {
@@ -3091,7 +3139,7 @@ int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail) {
 int launch_bse_pair(ldga_ctx* ctx, int32_t* d_fail) {
     const BseVariant* v = nullptr;
     const int nv = variants_of(ctx->Nnu, ctx->prec, &v);
-    int i = nv > 0 ? tuned_index(ctx->Nnu, ctx->prec) : 0;
+    int i = nv > 0 ? chosen_variant(ctx) : 0;
     if (i >= nv) i = 0;
     if (nv == 0 || !v[i].run_pair) {
         const int st = launch_bse(ctx, LDGA_CH_M, d_fail);
