@@ -2513,38 +2513,83 @@ __global__ void __launch_bounds__(T * T, MINB) k_bse_adj(const BseAdjArgs a) {
     for (int q = q0; q < q1; ++q) solve(q, blockIdx.y);
 }
 
-// Gamma_bar(w)[a, b] = -sum_q conj(y[q, a, w]) z[q, b, w], one CTA per (w, 32 x 32 output tile);
-// q is staged through shared memory in chunks, summed in a fixed order.
+// Gamma_bar(w)[a, b] = -sum_q conj(y[q, a, w]) z[q, b, w] on the FP64 tensor path (mma.sync m8n8k4, the sum over q
+// as its k index): one CTA per (8 rows a, w), all n columns b in NB tiles of 8; its 8 warps take every
+// eighth group of four q, reading both operands from global memory in fragment order (y and z have q
+// fastest: four consecutive q of one row are one 64-byte segment), and their accumulators are added in
+// warp order, so the result does not depend on timing.  Bound by the latency of a warp's operand loads
+// (four groups in flight).  2D 48^2, Nnu = 40 (325 q, 41 w): 71 us before with FP64 FMAs on 32 x 32 tiles
+// of 40 x 40 outputs staged through shared memory; 25 us.
+template <int NB>
 __global__ void __launch_bounds__(256) k_bse_gamma_grad(int nq, int n, const double2* __restrict__ y,
                                                         const double2* __restrict__ z, double2* __restrict__ gbar) {
-    constexpr int TQ = 16;
-    __shared__ double2 ys[TQ][32], zs[TQ][32];
-    const int w = blockIdx.z;
-    const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
-    const int ta = threadIdx.x & 31, tb = threadIdx.x >> 5;   // 32 x 8 threads, 4 outputs each
-    double2 acc[4] = {dmk(0, 0), dmk(0, 0), dmk(0, 0), dmk(0, 0)};
-    for (int qc = 0; qc < nq; qc += TQ) {
-        for (int e = threadIdx.x; e < TQ * 32; e += blockDim.x) {
-            const int qq = e / 32, jj = e % 32;
-            const int qi = qc + qq;
-            const bool ok = qi < nq;
-            ys[qq][jj] = (ok && a0 + jj < n) ? y[(size_t)qi + (size_t)nq * (a0 + jj + (size_t)n * w)] : dmk(0, 0);
-            zs[qq][jj] = (ok && b0 + jj < n) ? z[(size_t)qi + (size_t)nq * (b0 + jj + (size_t)n * w)] : dmk(0, 0);
+    __shared__ double4 part[8][32];
+    const int w = blockIdx.y, a0 = blockIdx.x * 8, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, t = lane & 3;
+    double re[NB][2], im[NB][2];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) re[b][0] = re[b][1] = im[b][0] = im[b][1] = 0.0;
+    const double2* yw = y + (size_t)nq * n * w;
+    const double2* zw = z + (size_t)nq * n * w;
+    const int steps = (nq + 3) / 4;
+    constexpr int U = NB <= 5 ? 4 : 2;             // groups of four q whose loads are in flight
+    const double2* ya = yw + (size_t)nq * min(a0 + g, n - 1);
+    const bool aok = a0 + g < n;
+    for (int s = warp; s < steps; s += 8 * U) {
+        double2 yv[U], zv[U][NB];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {              // addresses kept in range, values outside set to zero
+            const int q = 4 * (s + 8 * u) + t, qc = min(q, nq - 1);
+            const bool ok = q < nq;
+            yv[u] = ya[qc];
+            if (!ok || !aok) yv[u] = dmk(0.0, 0.0);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                zv[u][b] = zw[(size_t)qc + (size_t)nq * min(8 * b + g, n - 1)];
+                if (!ok || 8 * b + g >= n) zv[u][b] = dmk(0.0, 0.0);
+            }
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {         // conj(y) z
+                mma_f64(re[b], yv[u].x, zv[u][b].x);
+                mma_f64(im[b], yv[u].x, zv[u][b].y);
+                mma_f64(re[b], yv[u].y, zv[u][b].y);
+                mma_f64(im[b], -yv[u].y, zv[u][b].x);
+            }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        part[warp][lane] = make_double4(re[b][0], re[b][1], im[b][0], im[b][1]);
         __syncthreads();
+        if (tid < 64) {                            // element (row l / 4, column 2 (l mod 4) + e)
+            const int l = tid >> 1, e = tid & 1, aa = a0 + (l >> 2), bb = 8 * b + 2 * (l & 3) + e;
+            double sr = 0.0, si = 0.0;
 #pragma unroll
-        for (int qq = 0; qq < TQ; ++qq) {
-            const double2 ya = cconj(ys[qq][ta]);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) acc[r] = cadd(acc[r], cmul(ya, zs[qq][tb + 8 * r]));
+            for (int k = 0; k < 8; ++k) {
+                const double4 v = part[k][l];
+                sr += e ? v.y : v.x;
+                si += e ? v.w : v.z;
+            }
+            if (aa < n && bb < n) gbar[(size_t)aa + (size_t)n * (bb + (size_t)n * w)] = dmk(-sr, -si);
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int aa = a0 + ta, bb = b0 + tb + 8 * r;
-        if (aa < n && bb < n) gbar[(size_t)aa + (size_t)n * (bb + (size_t)n * w)] = cscale(acc[r], -1.0);
+}
+
+int launch_gamma_grad(ldga_ctx* ctx, const double2* y, const double2* z, double2* gbar) {
+    const int n = ctx->Nnu;
+    const dim3 grid((n + 7) / 8, ctx->Nw);
+    switch ((n + 7) / 8) {
+#define LDGA_GG(NB) \
+    case NB: k_bse_gamma_grad<NB><<<grid, 256, 0, ctx->stream>>>(ctx->Nq, n, y, z, gbar); break;
+        LDGA_GG(1) LDGA_GG(2) LDGA_GG(3) LDGA_GG(4) LDGA_GG(5) LDGA_GG(6) LDGA_GG(7) LDGA_GG(8)
+#undef LDGA_GG
+        default: return ctx_fail(ctx, LDGA_ERR_ARG, "BSE adjoint: fermionic box above 64");
     }
+    LDGA_LAUNCHED(ctx, "k_bse_gamma_grad");
+    return LDGA_OK;
 }
 
 template <int N, int T, int MINB>
@@ -2990,29 +3035,48 @@ __global__ void k_transpose_gamma(int n, int nw, const double2* __restrict__ src
     }
 }
 
-// one thread per (q, w): two sweeps over nu (q fastest in memory, so the warp's loads coalesce)
-__global__ void k_adj_rhs(const BseAdjArgs a) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;   // q + Nq w
-    if (e >= a.nq * a.nw) return;
-    const int q = e % a.nq, w = e / a.nq, n = a.nnu;
+// 32 q x 8 slices of nu per CTA (q fastest in memory, so a warp's loads coalesce); a thread keeps its PER
+// elements' 1/chi0 between the two sweeps (before: one thread per (q, w), 53 CTAs at 2D 48^2, every
+// reciprocal twice: 77 us at Nnu = 40, 41 w; 22 us)
+template <int PER>
+__global__ void __launch_bounds__(256) k_adj_rhs(const BseAdjArgs a) {
+    __shared__ double red[8][32];
+    const int tx = threadIdx.x & 31, sl = threadIdx.x >> 5, q = blockIdx.x * 32 + tx, w = blockIdx.y, n = a.nnu;
+    const bool own = q < a.nq;
+    const size_t e = (size_t)(own ? q : 0) + (size_t)a.nq * w;
     const double f = 1.0 + a.s * a.U * a.chi[e], rf = 1.0 / f;
+    double2 d[PER], gb[PER];
     double s1 = 0.0;
-    for (int i = 0; i < n; ++i) {
-        const size_t ci = (size_t)q + (size_t)a.nq * (i + (size_t)n * w);
-        const double2 c0 = a.chi0[ci];
-        const double2 y = cscale(cmul(a.gam[ci], c0), f);
-        a.ybuf[ci] = y;
-        if (a.gam_bar) {
-            const double2 gb = a.gam_bar[ci], yd = cmul(y, cinv(c0));
-            s1 += gb.x * yd.x + gb.y * yd.y;             // Re(conj(gb) y d)
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = sl + 8 * k;
+        d[k] = gb[k] = dmk(0.0, 0.0);
+        if (own && i < n) {
+            const size_t ci = (size_t)q + (size_t)a.nq * (i + (size_t)n * w);
+            const double2 c0 = a.chi0[ci];
+            const double2 y = cscale(cmul(a.gam[ci], c0), f);
+            a.ybuf[ci] = y;
+            d[k] = cinv(c0);
+            if (a.gam_bar) {
+                gb[k] = a.gam_bar[ci];
+                const double2 yd = cmul(y, d[k]);
+                s1 += gb[k].x * yd.x + gb[k].y * yd.y;             // Re(conj(gb) y d)
+            }
         }
     }
-    const double xbar = (a.chi_bar ? a.chi_bar[e] : 0.0) - a.s * a.U * rf * rf * s1;
-    for (int i = 0; i < n; ++i) {
-        const size_t ci = (size_t)q + (size_t)a.nq * (i + (size_t)n * w);
-        double2 yb = make_double2(xbar / (a.beta * a.beta), 0.0);
-        if (a.gam_bar) yb = cadd(yb, cmul(cconj(cscale(cinv(a.chi0[ci]), rf)), a.gam_bar[ci]));
-        a.zbuf[ci] = cconj(yb);
+    red[sl][tx] = s1;
+    __syncthreads();
+    s1 = 0.0;
+    for (int k = 0; k < 8; ++k) s1 += red[k][tx];
+    const double xbar = (own && a.chi_bar ? a.chi_bar[e] : 0.0) - a.s * a.U * rf * rf * s1;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = sl + 8 * k;
+        if (own && i < n) {
+            double2 yb = make_double2(xbar / (a.beta * a.beta), 0.0);
+            if (a.gam_bar) yb = cadd(yb, cmul(cconj(cscale(d[k], rf)), gb[k]));
+            a.zbuf[(size_t)q + (size_t)a.nq * (i + (size_t)n * w)] = cconj(yb);
+        }
     }
 }
 
@@ -3195,8 +3259,7 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
         }
         k_transpose_gamma<<<2 * 148, 256, 0, ctx->stream>>>(N, ctx->Nw, ctx->d_Gamma[channel], ctx->d_gamma_t);
         LDGA_LAUNCHED(ctx, "k_transpose_gamma");
-        const int nqw = ctx->Nq * ctx->Nw;
-        k_adj_rhs<<<(nqw + 255) / 256, 256, 0, ctx->stream>>>(a);
+        k_adj_rhs<N / 8><<<dim3((ctx->Nq + 31) / 32, ctx->Nw), 256, 0, ctx->stream>>>(a);
         LDGA_LAUNCHED(ctx, "k_adj_rhs");
         BseArgs b = bse_args(ctx, channel);
         b.Gamma = ctx->d_gamma_t;
@@ -3237,10 +3300,8 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
     }
     }
     if (st != LDGA_OK) return st;
-    const int n = ctx->Nnu;
-    dim3 g2((n + 31) / 32, (n + 31) / 32, ctx->Nw);
-    k_bse_gamma_grad<<<g2, 256, 0, ctx->stream>>>(ctx->Nq, n, ybuf, zbuf, gamma_bar);
-    LDGA_LAUNCHED(ctx, "k_bse_gamma_grad");
+    st = launch_gamma_grad(ctx, ybuf, zbuf, gamma_bar);
+    if (st != LDGA_OK) return st;
     k_count_flags<<<148, 256, 0, ctx->stream>>>(ctx->d_flags, ctx->Nq * ctx->Nw, d_fail);
     LDGA_LAUNCHED(ctx, "k_count_flags");
     return LDGA_OK;

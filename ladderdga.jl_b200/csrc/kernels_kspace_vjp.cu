@@ -103,21 +103,25 @@ __global__ void __launch_bounds__((kThr<DIM, N, false>), (kMinB<DIM, N, false>))
     }
 }
 
-// s̄ = U Σ_{q,n} Im(Sbar(q, n)) / ν_n, one CTA, fixed order
-__global__ void __launch_bounds__(256) k_vjp_tail(int nq, int numax, double beta, double U,
+// s̄ = U Σ_{q,n} Im(Sbar(q, n)) / ν_n, one CTA, fixed order: a warp takes whole n, four loads in flight
+// (256 threads with a division per element 16 us at 325 q x 20 ν; 5 us)
+__global__ void __launch_bounds__(1024) k_vjp_tail(int nq, int numax, double beta, double U,
                                                    const double2* __restrict__ sbar, double* __restrict__ out) {
-    __shared__ double red[8];
+    __shared__ double red[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double acc = 0.0;
-    for (int e = threadIdx.x; e < nq * numax; e += blockDim.x) {
-        const int n = e / nq;
-        acc += sbar[e].y / ((2.0 * n + 1.0) * M_PI / beta);
+    for (int n = warp; n < numax; n += 32) {
+        double s = 0.0;
+#pragma unroll 4
+        for (int q = lane; q < nq; q += 32) s += sbar[(size_t)n * nq + q].y;
+        acc += s / ((2.0 * n + 1.0) * M_PI / beta);
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    if (lane == 0) red[warp] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
         double r = 0.0;
-        for (int i = 0; i < 8; ++i) r += red[i];
+        for (int i = 0; i < 32; ++i) r += red[i];
         out[0] = U * r;
     }
 }
@@ -258,16 +262,30 @@ __global__ void __launch_bounds__((kThr<DIM, N, false>), (kMinB<DIM, N, false>))
     }
 }
 
-// Ĝ̄[f][q] = Σ_{j in list(f)} rows[idx[j]][q], CSR over the fft_range frequencies, fixed order
-__global__ void __launch_bounds__(256) k_ghat_gather(int nf, int nq, const int32_t* __restrict__ start,
+// Ĝ̄[f][q] = Σ_{j in list(f)} rows[idx[j]][q], CSR over the fft_range frequencies: 32 q x 8 slices of the list per
+// CTA, eight rows of a slice in flight, the slices added in order (one thread per (f, q) walked its whole list
+// of up to about 120 rows: 49 us at 2D 48^2, Nν = 40, 41 ω; 8 us)
+__global__ void __launch_bounds__(256) k_ghat_gather(int nq, const int32_t* __restrict__ start,
                                                       const int32_t* __restrict__ idx, const double2* __restrict__ rows,
                                                       double2* __restrict__ gbar) {
-    const size_t n = (size_t)nf * nq;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int f = (int)(e / nq), q = (int)(e % nq);
-        double2 acc = make_double2(0.0, 0.0);
-        for (int j = start[f]; j < start[f + 1]; ++j) acc = cadd(acc, rows[(size_t)idx[j] * nq + q]);
-        gbar[e] = acc;
+    __shared__ double2 red[8][32];
+    const int tx = threadIdx.x & 31, sl = threadIdx.x >> 5, q = blockIdx.x * 32 + tx, f = blockIdx.y;
+    const int j0 = start[f], j1 = start[f + 1];
+    double2 acc = make_double2(0.0, 0.0);
+    if (q < nq)
+        for (int j = j0 + sl; j < j1; j += 64) {
+            double2 r[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                r[k] = j + 8 * k < j1 ? rows[(size_t)idx[j + 8 * k] * nq + q] : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc = cadd(acc, r[k]);
+        }
+    red[sl][tx] = acc;
+    __syncthreads();
+    if (sl == 0 && q < nq) {
+        for (int k = 1; k < 8; ++k) acc = cadd(acc, red[k][tx]);
+        gbar[(size_t)f * nq + q] = acc;
     }
 }
 
@@ -347,7 +365,7 @@ int run_gloc_vjp(ldga_ctx* ctx, const double2* chi0_bar, const double2* sbar, in
                                                    rows + (size_t)2 * nbub * ctx->Nq, np);
         LDGA_LAUNCHED(ctx, "k_eom_gvjp");
     }
-    k_ghat_gather<<<2 * 148, 256, 0, ctx->stream>>>(ctx->Nf, ctx->Nq, start, idx, rows, gbar_hat);
+    k_ghat_gather<<<dim3((ctx->Nq + 31) / 32, ctx->Nf), 256, 0, ctx->stream>>>(ctx->Nq, start, idx, rows, gbar_hat);
     LDGA_LAUNCHED(ctx, "k_ghat_gather");
     {
         const int np = pairs_per_cta<DIM, N>(ctx->Nf);
@@ -391,7 +409,7 @@ int run_eom_vjp(ldga_ctx* ctx, int numax, double lam_m, double lam_d, int tc, co
         LDGA_LAUNCHED(ctx, "k_eom_vjp");
     }
     if (tc) {
-        k_vjp_tail<<<1, 256, 0, ctx->stream>>>(ctx->Nq, numax, ctx->mp.beta, ctx->mp.U, sbar, ctx->d_red + 60);
+        k_vjp_tail<<<1, 1024, 0, ctx->stream>>>(ctx->Nq, numax, ctx->mp.beta, ctx->mp.U, sbar, ctx->d_red + 60);
         LDGA_LAUNCHED(ctx, "k_vjp_tail");
     }
     const double tail_w = tc ? 1.0 / (ctx->mp.beta * (double)ctx->Nk) : 0.0;
