@@ -13,7 +13,7 @@ struct BseArgs {
     double2* gam;           // [Nq, Nnu, Nw]
     int32_t* flags;         // [Nq, Nw]
     unsigned long long* stats = nullptr;   // [2] residual passes and warps of 8 q (may be null)
-    // the iterations: a flagged matrix is also appended (q + Nq w) to fail_list at atomicAdd(fail_count)
+    // a flagged matrix is also appended (q + Nq w) to fail_list at atomicAdd(fail_count)
     int32_t* fail_list = nullptr;
     int32_t* fail_count = nullptr;
     int max_sweeps = 40;    // residual sweeps of an iteration before a q is flagged

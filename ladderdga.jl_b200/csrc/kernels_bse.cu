@@ -100,6 +100,16 @@ __device__ __forceinline__ void named_barrier(int id, int nthreads) {
 
 __device__ __forceinline__ double2 dmk(double r, double i) { return make_double2(r, i); }
 
+// The channel of a two-channel launch (blockIdx.z): chi0, the q order and the sizes are shared.
+__device__ __forceinline__ BseArgs pick_channel(const BseArgs& m, const BseArgs& d) {
+    BseArgs a = m;
+    if (blockIdx.z) {
+        a.s = d.s; a.Gamma = d.Gamma; a.chi = d.chi; a.gam = d.gam; a.flags = d.flags;
+        a.fail_list = d.fail_list; a.fail_count = d.fail_count;
+    }
+    return a;
+}
+
 // Group-wide reduction of NV values (op 1: max, 0: sum) over the group's G threads, fixed order.
 // red: per-group shared scratch [NV * (G/32)].  Result in every thread of the group.
 template <int NV, int G>
@@ -391,6 +401,7 @@ __global__ void __launch_bounds__(TR * TC * MPC, MINB) k_bse_tile(const BseArgs 
         if (t == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
+            if (!ok && a.fail_list) a.fail_list[atomicAdd(a.fail_count, 1)] = q + a.nq * w;
         }
         const double f = 1.0 + a.s * a.U * chi;
 #pragma unroll
@@ -446,8 +457,9 @@ struct LuSmem {
         (2 * RW + 2 * CW + N + N + N) * sizeof(double2) + 8 * (G / 32) * sizeof(double) + 16;
 };
 
-template <int N, int T, int MPC, int MINB, bool GSM, bool LA, bool PAD>
-__global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a) {
+template <int N, int T, int MPC, int MINB, bool GSM, bool LA, bool PAD, bool PAIR>
+__global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a_m, const BseArgs a_d) {
+    const BseArgs a = PAIR ? pick_channel(a_m, a_d) : a_m;
     using LS = LuSmem<N, T>;
     constexpr int RT = LS::RT, NC = LS::NC, G = LS::G;
     constexpr int CT = (NC + T - 1) / T;
@@ -703,6 +715,7 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a) {
         if (t == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
+            if (!ok && a.fail_list) a.fail_list[atomicAdd(a.fail_count, 1)] = q + a.nq * w;
         }
         const double rf = 1.0 / (1.0 + a.s * a.U * chi);
 #pragma unroll
@@ -1000,6 +1013,7 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu32(const BseArgs a)
         if (t == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
+            if (!ok && a.fail_list) a.fail_list[atomicAdd(a.fail_count, 1)] = q + a.nq * w;
         }
         const double rf = 1.0 / (1.0 + a.s * a.U * chi);
         for (int i = t; i < N; i += G) {
@@ -1044,8 +1058,9 @@ struct Warp32Smem {
         (2 * CT * TC + 2 * RT * TR) * sizeof(float4) + 2 * RT * TR * sizeof(float2) + 2 * N * sizeof(double2);
 };
 
-template <int N, int TR, int TC, int WPC, int MINB>
-__global__ void __launch_bounds__(32 * WPC, MINB) k_bse_warp32(const BseArgs a) {
+template <int N, int TR, int TC, int WPC, int MINB, bool PAIR>
+__global__ void __launch_bounds__(32 * WPC, MINB) k_bse_warp32(const BseArgs a_m, const BseArgs a_d) {
+    const BseArgs a = PAIR ? pick_channel(a_m, a_d) : a_m;
     using WS = Warp32Smem<N, TR, TC>;
     constexpr int RT = WS::RT, CT = WS::CT;
     constexpr int NH = TR / TC;                           // tile columns per tile row
@@ -1326,6 +1341,7 @@ __global__ void __launch_bounds__(32 * WPC, MINB) k_bse_warp32(const BseArgs a) 
         if (lane == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
+            if (!ok && a.fail_list) a.fail_list[atomicAdd(a.fail_count, 1)] = q + a.nq * w;
         }
         const double rf = 1.0 / (1.0 + a.s * a.U * chi);
         for (int i = lane; i < N; i += 32) {
@@ -2700,7 +2716,7 @@ __device__ bool pivot_solve(const BseArgs& a, int lin, double2* B, double* red, 
 }
 
 __global__ void __launch_bounds__(256) k_bse_lu_pivot(const BseArgs a, const int32_t* list, int count,
-                                                       const int32_t* count_dev, double2* gscratch) {
+                                                       const int32_t* count_dev, double2* gscratch, int32_t* d_fail) {
     extern __shared__ double2 sm[];
     const int N = a.nnu;
     double* red = reinterpret_cast<double*>(sm);                      // [64]
@@ -2708,7 +2724,10 @@ __global__ void __launch_bounds__(256) k_bse_lu_pivot(const BseArgs a, const int
     double2* B = gscratch ? gscratch + (size_t)blockIdx.x * N * (N + 1)   // [N][N+1] row-major, rhs last
                           : reinterpret_cast<double2*>(piv_s + 4);
     if (count_dev) count = count_dev[0];
-    for (int item = blockIdx.x; item < count; item += gridDim.x) pivot_solve(a, list ? list[item] : item, B, red, piv_s);
+    for (int item = blockIdx.x; item < count; item += gridDim.x) {
+        const bool ok = pivot_solve(a, list ? list[item] : item, B, red, piv_s);
+        if (threadIdx.x == 0 && !ok) atomicAdd(d_fail, 1);
+    }
 }
 
 // Both channels' flagged matrices of a two-channel preconditioned solve in one launch: the lists the
@@ -2732,14 +2751,6 @@ __global__ void __launch_bounds__(256) k_bse_lu_pivot_pair(const BseArgs am, con
     }
 }
 
-__global__ void k_compact_flags(const int32_t* flags, int n, int32_t* list, int32_t* count) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        if (flags[e] != 0) {
-            const int pos = atomicAdd(count, 1);
-            list[pos] = e;
-        }
-    }
-}
 __global__ void k_count_flags(const int32_t* flags, int n, int32_t* count) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
         if (flags[e] != 0) atomicAdd(count, 1);
@@ -2764,21 +2775,35 @@ int run_tile(ldga_ctx* ctx, const BseArgs& a0) {
     return LDGA_OK;
 }
 
-template <int N, int T, int MPC, int MINB, bool GSM = true, bool LA = LDGA_LU_LOOKAHEAD, bool PAD = false>
-int run_lu(ldga_ctx* ctx, const BseArgs& a0) {
-    BseArgs a = a0;
+// q per CTA: up to four per matrix group, fewer while the launch has less than eight CTAs per SM
+template <bool PAIR>
+int lu_chunk(const BseArgs& a, int per) {
+    int chunk = 4 * per;
+    while (chunk > per && (long)((a.nq + chunk - 1) / chunk) * a.nw * (PAIR ? 2 : 1) < 8 * 148) chunk -= per;
+    return chunk;
+}
+
+template <int N, int T, int MPC, int MINB, bool GSM, bool LA, bool PAD, bool PAIR>
+int run_lu_impl(ldga_ctx* ctx, BseArgs a, BseArgs d) {
     const int threads = T * T * MPC;
     const size_t sm = (GSM ? (size_t)N * N * sizeof(double2) : 0) + MPC * LuSmem<N, T>::bytes;
-    auto kern = k_bse_lu<N, T, MPC, MINB, GSM, LA, PAD>;
+    auto kern = k_bse_lu<N, T, MPC, MINB, GSM, LA, PAD, PAIR>;
     LDGA_CUDA(ctx, set_smem(ctx, kern, sm));
-    int chunk = 4 * MPC;
-    while (chunk > MPC && (long)((a.nq + chunk - 1) / chunk) * a.nw < 8 * 148) chunk -= MPC;
-    a.qchunk = chunk;
-    dim3 grid((a.nq + chunk - 1) / chunk, a.nw);
+    a.qchunk = d.qchunk = lu_chunk<PAIR>(a, MPC);
+    dim3 grid((a.nq + a.qchunk - 1) / a.qchunk, a.nw, PAIR ? 2 : 1);
     StageTimer st_(ctx, LDGA_STAGE_BSE);
-    kern<<<grid, threads, sm, ctx->stream>>>(a);
+    kern<<<grid, threads, sm, ctx->stream>>>(a, d);
     LDGA_LAUNCHED(ctx, "k_bse_lu");
     return LDGA_OK;
+}
+
+template <int N, int T, int MPC, int MINB, bool GSM = true, bool LA = LDGA_LU_LOOKAHEAD, bool PAD = false>
+int run_lu(ldga_ctx* ctx, const BseArgs& a) {
+    return run_lu_impl<N, T, MPC, MINB, GSM, LA, PAD, false>(ctx, a, a);
+}
+template <int N, int T, int MPC, int MINB, bool GSM = true, bool LA = LDGA_LU_LOOKAHEAD, bool PAD = false>
+int run_lu_pair(ldga_ctx* ctx, const BseArgs& a_m, const BseArgs& a_d) {
+    return run_lu_impl<N, T, MPC, MINB, GSM, LA, PAD, true>(ctx, a_m, a_d);
 }
 
 template <int N, int T, int MPC, int MINB, bool GSM = true>
@@ -2798,21 +2823,27 @@ int run_lu32(ldga_ctx* ctx, const BseArgs& a0) {
     return LDGA_OK;
 }
 
-template <int N, int TR, int TC, int WPC, int MINB>
-int run_warp32(ldga_ctx* ctx, const BseArgs& a0) {
-    BseArgs a = a0;
+template <int N, int TR, int TC, int WPC, int MINB, bool PAIR>
+int run_warp32_impl(ldga_ctx* ctx, BseArgs a, BseArgs d) {
     const int threads = 32 * WPC;
     const size_t sm = (size_t)N * N * sizeof(double2) + WPC * Warp32Smem<N, TR, TC>::bytes;
-    auto kern = k_bse_warp32<N, TR, TC, WPC, MINB>;
+    auto kern = k_bse_warp32<N, TR, TC, WPC, MINB, PAIR>;
     LDGA_CUDA(ctx, set_smem(ctx, kern, sm));
-    int chunk = 4 * WPC;
-    while (chunk > WPC && (long)((a.nq + chunk - 1) / chunk) * a.nw < 8 * 148) chunk -= WPC;
-    a.qchunk = chunk;
-    dim3 grid((a.nq + chunk - 1) / chunk, a.nw);
+    a.qchunk = d.qchunk = lu_chunk<PAIR>(a, WPC);
+    dim3 grid((a.nq + a.qchunk - 1) / a.qchunk, a.nw, PAIR ? 2 : 1);
     StageTimer st_(ctx, LDGA_STAGE_BSE);
-    kern<<<grid, threads, sm, ctx->stream>>>(a);
+    kern<<<grid, threads, sm, ctx->stream>>>(a, d);
     LDGA_LAUNCHED(ctx, "k_bse_warp32");
     return LDGA_OK;
+}
+
+template <int N, int TR, int TC, int WPC, int MINB>
+int run_warp32(ldga_ctx* ctx, const BseArgs& a) {
+    return run_warp32_impl<N, TR, TC, WPC, MINB, false>(ctx, a, a);
+}
+template <int N, int TR, int TC, int WPC, int MINB>
+int run_warp32_pair(ldga_ctx* ctx, const BseArgs& a_m, const BseArgs& a_d) {
+    return run_warp32_impl<N, TR, TC, WPC, MINB, true>(ctx, a_m, a_d);
 }
 
 #include "bse_jacobi.cuh"
@@ -2867,9 +2898,10 @@ struct BseVariant {
 };
 
 #define LDGA_SMALL_BOX(N)                                                                              \
-    const BseVariant fp64_##N[] = {{&run_lu<N, 8, 1, 2>, "lu8:2"}, {&run_lu<N, 8, 1, 4>, "lu8:4"},     \
+    const BseVariant fp64_##N[] = {{&run_lu<N, 8, 1, 2>, "lu8:2", &run_lu_pair<N, 8, 1, 2>},           \
+                                   {&run_lu<N, 8, 1, 4>, "lu8:4"},                                     \
                                    {&run_lu<N, 8, 1, 8>, "lu8:8"}};                                     \
-    const BseVariant mixed_##N[] = {{&run_warp32<N, 8, 4, 4, 1>, "warp:1"},                            \
+    const BseVariant mixed_##N[] = {{&run_warp32<N, 8, 4, 4, 1>, "warp:1", &run_warp32_pair<N, 8, 4, 4, 1>}, \
                                     {&run_warp32<N, 8, 4, 4, 3>, "warp:3"}};                           \
     const BseVariant inv_##N[] = {{&run_tile<N, 8, 8, 2, 1, double, LDGA_PREC_FP64_INV>, "gj8x2"}};
 LDGA_SMALL_BOX(4)
@@ -2884,9 +2916,11 @@ LDGA_SMALL_BOX(12)
 // on tcgen05) on tiles of NP >= N rows, NP a multiple of 8, as a candidate: with few q per ω its
 // groups are wide, so the autotuner decides
 #define LDGA_ITER_BOX(N, LPQ, MINB, NP, MINB_TC, TCNAME)                                                \
-    const BseVariant fp64_##N[] = {{&run_lu<N, 8, 1, 2>, "lu8:2"}, {&run_lu<N, 8, 1, 4>, "lu8:4"},     \
+    const BseVariant fp64_##N[] = {{&run_lu<N, 8, 1, 2>, "lu8:2", &run_lu_pair<N, 8, 1, 2>},           \
+                                   {&run_lu<N, 8, 1, 4>, "lu8:4"},                                     \
                                    {&run_lu<N, 8, 1, 8>, "lu8:8"}};                                     \
-    const BseVariant mixed_##N[] = {{&run_warp32<N, 8, 4, 4, 1>, "warp:1"}, {&run_warp32<N, 8, 4, 4, 3>, "warp:3"}, \
+    const BseVariant mixed_##N[] = {{&run_warp32<N, 8, 4, 4, 1>, "warp:1", &run_warp32_pair<N, 8, 4, 4, 1>}, \
+                                    {&run_warp32<N, 8, 4, 4, 3>, "warp:3"},                            \
                                     {&run_iter<N, LPQ, MINB>, "iter"},                                 \
                                     {&run_iter<NP, 8, MINB_TC, 2, true, true, true, true, true, N>, TCNAME, \
                                      &run_iter_pair<NP, 8, MINB_TC, 2, true, true, true, true, true, N>}}; \
@@ -2896,7 +2930,7 @@ LDGA_ITER_BOX(20, 4, 4, 24, 4, "iter8x2dm2ns24:4")
 LDGA_ITER_BOX(30, 4, 3, 32, 3, "iter8x2dm2ns32:3")
 #undef LDGA_ITER_BOX
 constexpr int kIter30 = 3;   // the tensor-core iteration in mixed_30
-const BseVariant fp64_40[] = {{&run_lu<40, 8, 1, 6>, "lu8:6"}, {&run_lu<40, 8, 1, 4>, "lu8:4"},
+const BseVariant fp64_40[] = {{&run_lu<40, 8, 1, 6>, "lu8:6", &run_lu_pair<40, 8, 1, 6>}, {&run_lu<40, 8, 1, 4>, "lu8:4"},
                               {&run_lu<40, 8, 1, 5>, "lu8:5"}};
 // the default: the group inverse by Newton-Schulz on tcgen05 tensor cores (Gauss-Jordan as its fallback)
 const BseVariant mixed_40[] = {{&run_iter<40, 8, 3, 2, true, true, true, true, true>, "iter8x2dm2ns:3",
@@ -2910,7 +2944,7 @@ const BseVariant mixed_40[] = {{&run_iter<40, 8, 3, 2, true, true, true, true, t
                                {&run_iter<40, 8, 2>, "iter8:2"}, {&run_iter<40, 4, 3>, "iter"},
                                {&run_warp32<40, 8, 4, 4, 3>, "warp:3"}, {&run_warp32<40, 8, 4, 4, 2>, "warp:2"}};
 const BseVariant inv_40[] = {{&run_tile<40, 8, 8, 2, 1, double, LDGA_PREC_FP64_INV>, "gj8x2"}};
-const BseVariant fp64_60[] = {{&run_lu<60, 16, 1, 2>, "lu16:2"}, {&run_lu<60, 16, 1, 1>, "lu16:1"},
+const BseVariant fp64_60[] = {{&run_lu<60, 16, 1, 2>, "lu16:2", &run_lu_pair<60, 16, 1, 2>}, {&run_lu<60, 16, 1, 1>, "lu16:1"},
                               {&run_lu<60, 16, 1, 3>, "lu16:3"}};
 // MIXED may pick any configuration whose results meet the FP64 backward-error bound, the FP64 LU
 // included: at Nν = 60 and 120 that is the fastest one measured
@@ -2936,7 +2970,8 @@ const BseVariant mixed_120[] = {{&run_jacobi<120, 32, 4, true>, "jac", &run_jaco
 // pivoted kernel (a 128 x 129 register tile spills, Gamma(w) outgrows shared memory).
 template <int N, int T, int MINB>
 constexpr BseVariant padded_lu(const char* name) {
-    return {&run_lu<N, T, 1, MINB, true, LDGA_LU_LOOKAHEAD, true>, name};
+    return {&run_lu<N, T, 1, MINB, true, LDGA_LU_LOOKAHEAD, true>, name,
+            &run_lu_pair<N, T, 1, MINB, true, LDGA_LU_LOOKAHEAD, true>};
 }
 const BseVariant padded_lus[] = {padded_lu<8, 8, 8>("lu8p8"),     padded_lu<16, 8, 8>("lu8p16"),
                                  padded_lu<24, 8, 8>("lu8p24"),   padded_lu<32, 8, 6>("lu8p32"),
@@ -3154,52 +3189,44 @@ int bse_run_variant(ldga_ctx* ctx, int channel, int i) {
     return v[i].run(ctx, bse_args(ctx, channel));
 }
 
+// One channel: the configuration appends the matrices it leaves above its backward-error bound to d_list (count
+// in d_count[0]), a grid-stride pivoted launch re-solves the list (zero work when it is empty) and counts
+// into *d_fail what stays non-finite.  Appending takes the place of two passes over the flags around the
+// pivoted launch: a call at Nnu = 40 on 32^3 takes 590 us, 610 us with them, at Nnu = 34 on 12^3 in FP64
+// 271 us (290 us).
 int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail) {
-    const BseArgs a = bse_args(ctx, channel);
+    BseArgs a = bse_args(ctx, channel);
     const int n = ctx->Nq * shard_nw(ctx);
-    int st = LDGA_OK;
-    bool generic = false;
-    {
-        const BseVariant* v = nullptr;
-        const int nv = variants_of(ctx->Nnu, ctx->prec, &v);
-        if (nv > 0) {
-            int i = chosen_variant(ctx);
-            if (i >= nv) i = 0;
-            st = v[i].run(ctx, a);
-        } else {
-            generic = true;
-        }
+    const BseVariant* v = nullptr;
+    const int nv = variants_of(ctx->Nnu, ctx->prec, &v);
+    if (nv > 0) {
+        int i = chosen_variant(ctx);
+        if (i >= nv) i = 0;
+        LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count, 0, sizeof(int32_t), ctx->stream));
+        a.fail_list = ctx->d_list;
+        a.fail_count = ctx->d_count;
+        const int st = v[i].run(ctx, a);
+        if (st != LDGA_OK) return st;
     }
-    if (st != LDGA_OK) return st;
     const bool in_hbm = bse_pivot_smem(ctx->Nnu) > LDGA_PIVOT_SMEM_MAX;
     if (in_hbm && !ctx->d_pivot_scratch) return ctx_fail(ctx, LDGA_ERR_ARG, "pivoted BSE scratch missing");
     const size_t smp = in_hbm ? 64 * sizeof(double) + 16 : bse_pivot_smem(ctx->Nnu);
     double2* gscr = in_hbm ? ctx->d_pivot_scratch : nullptr;
     LDGA_CUDA(ctx, set_smem(ctx, k_bse_lu_pivot, smp));
-    if (generic) {
-        StageTimer st_(ctx, LDGA_STAGE_BSE_FALLBACK);
-        k_bse_lu_pivot<<<LDGA_PIVOT_GRID, 256, smp, ctx->stream>>>(a, nullptr, n, nullptr, gscr);
-        LDGA_LAUNCHED(ctx, "k_bse_lu_pivot");
-    } else {
-        // flagged matrices: compacted on the device, re-solved by a grid-stride pivoted kernel that reads
-        // the count from device memory (zero work when nothing was flagged)
-        LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count, 0, sizeof(int32_t), ctx->stream));
-        k_compact_flags<<<148, 256, 0, ctx->stream>>>(a.flags, n, ctx->d_list, ctx->d_count);
-        LDGA_LAUNCHED(ctx, "k_compact_flags");
-        StageTimer st_(ctx, LDGA_STAGE_BSE_FALLBACK);
-        k_bse_lu_pivot<<<LDGA_PIVOT_GRID, 256, smp, ctx->stream>>>(a, ctx->d_list, 0, ctx->d_count, gscr);
-        LDGA_LAUNCHED(ctx, "k_bse_lu_pivot");
-    }
-    // matrices that stayed non-finite after the pivoted solve, accumulated into *d_fail
-    k_count_flags<<<148, 256, 0, ctx->stream>>>(a.flags, n, d_fail);
-    LDGA_LAUNCHED(ctx, "k_count_flags");
+    StageTimer st_(ctx, LDGA_STAGE_BSE_FALLBACK);
+    if (nv > 0) k_bse_lu_pivot<<<LDGA_PIVOT_GRID, 256, smp, ctx->stream>>>(a, ctx->d_list, 0, ctx->d_count, gscr, d_fail);
+    else k_bse_lu_pivot<<<LDGA_PIVOT_GRID, 256, smp, ctx->stream>>>(a, nullptr, n, nullptr, gscr, d_fail);
+    LDGA_LAUNCHED(ctx, "k_bse_lu_pivot");
     return LDGA_OK;
 }
 
 // Both channels of the chain: one launch of the tuned configuration when it has a two-channel form
 // (channel d flags into d_flags2); the matrices it leaves above its backward-error bound are appended
 // to one list per channel (counts in d_count[2], d_count[3], zeroed by the caller with d_fail) and
-// re-solved by one pivoted launch over both lists.  Otherwise launch_bse for m, then d.
+// re-solved by one pivoted launch over both lists.  Otherwise launch_bse for m, then d.  Every default
+// but FP64_INV's has the form: at the small boxes one channel alone leaves most of the chip idle and its
+// time is the chain of one matrix's elimination (Nnu = 20 on 16^2: 945 warps; the whole chain 125 us,
+// 140 us with the channels one after the other).
 int launch_bse_pair(ldga_ctx* ctx, int32_t* d_fail) {
     const BseVariant* v = nullptr;
     const int nv = variants_of(ctx->Nnu, ctx->prec, &v);

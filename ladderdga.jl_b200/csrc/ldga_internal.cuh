@@ -104,7 +104,7 @@ struct ldga_ctx {
     double* d_red = nullptr;       // reduction scratch
     int32_t* d_flags = nullptr;    // BSE fallback flags [Nq*Nw]
     int32_t* d_flags2 = nullptr;   // the d channel's flags when both channels run in one launch
-    int32_t* d_list = nullptr;     // compacted fallback list (the m channel's list of a pair launch)
+    int32_t* d_list = nullptr;     // matrices left to the pivoted solve (the m channel's list of a pair launch)
     int32_t* d_list2 = nullptr;    // the d channel's list of a pair launch
     double2* d_gamma_t = nullptr;  // MIXED BSE adjoint: Gamma(w) transposed [Nnu, Nnu, Nw]
     int32_t* d_count = nullptr;
@@ -219,7 +219,7 @@ int require_unsharded(ldga_ctx* ctx, const char* what);
 
 bool bse_has_fast_path(int nnu);
 // BSE kernel configurations (autotuning): count and name per (Nν, precision), the chosen index,
-// and one uncompacted launch of configuration i on the channel's current inputs.
+// and one launch of configuration i on the channel's current inputs.
 int bse_variant_count(int nnu, int prec);
 const char* bse_variant_name(int nnu, int prec, int i);
 int bse_tuned_variant(int nnu, int prec);
