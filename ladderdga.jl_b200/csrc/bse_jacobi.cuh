@@ -305,7 +305,7 @@ k_bse_jacobi(const BseArgs a_m, const BseArgs a_d) {
         const double x = (red[q] + red[kJacQ + q] + red[2 * kJacQ + q]) / (a.beta * a.beta);
         const size_t o = (size_t)(q0 + q) + (size_t)a.nq * w;
         a.chi[o] = x;
-        const bool ok = conv[q] != 0;
+        const bool ok = conv[q] != 0 && isfinite(x);
         a.flags[o] = ok ? 0 : 1;
         if (!ok && a.fail_list) a.fail_list[atomicAdd(a.fail_count, 1)] = (int32_t)o;
     }

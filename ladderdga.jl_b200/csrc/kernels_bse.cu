@@ -32,7 +32,7 @@
 //                       FP32 multipliers), or the FP64 elimination.
 // No pivoting is done in the fast path.  Every solution is verified by its FP64 backward error
 // |1 - B y|_inf / (|B|_inf |y|_inf + 1); a matrix above 1e-12 (1e-14 for the preconditioned
-// iteration), or with a non-finite y, is flagged
+// iteration), or with a non-finite y (seen in its sum chi: the maxima of the error drop a NaN), is flagged
 // and re-solved by a partial-pivoting FP64 LU kernel, which is also the path for boxes above Nν = 112 (but
 // 120); other box sizes without kernels of their own run on the next tile.
 #include <cmath>
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(TR * TC * MPC, MINB) k_bse_tile(const BseArgs 
 
         // ---- chi and gamma
         const double chi = ysum / (a.beta * a.beta);
-        const bool ok = isfinite(berr) && berr <= 1e-12;
+        const bool ok = isfinite(chi) && isfinite(berr) && berr <= 1e-12;
         if (t == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a_m,
 
         // ---- chi and gamma = y / (chi0 (1 + s U chi))
         const double chi = st[3] / (a.beta * a.beta);
-        const bool ok = isfinite(berr) && berr <= 1e-12;
+        const bool ok = isfinite(chi) && isfinite(berr) && berr <= 1e-12;
         if (t == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
@@ -1009,7 +1009,7 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu32(const BseArgs a)
 
         // ---- chi and gamma = y / (chi0 (1 + s U chi))
         const double chi = ysum / (a.beta * a.beta);
-        const bool ok = isfinite(berr) && berr <= 1e-12;
+        const bool ok = isfinite(chi) && isfinite(berr) && berr <= 1e-12;
         if (t == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
@@ -1337,7 +1337,7 @@ __global__ void __launch_bounds__(32 * WPC, MINB) k_bse_warp32(const BseArgs a_m
 
         // ---- chi and gamma = y / (chi0 (1 + s U chi))
         const double chi = ysum / (a.beta * a.beta);
-        const bool ok = isfinite(berr) && berr <= 1e-12;
+        const bool ok = isfinite(chi) && isfinite(berr) && berr <= 1e-12;
         if (lane == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
@@ -2262,7 +2262,7 @@ __global__ void __launch_bounds__(kIterQ * LPQ / QPL, MINB) k_bse_iter(const Bse
         if (ql >= nvalid) continue;
         const int q = pw[ql];
         const double chi = sx / (a.beta * a.beta);
-        const bool ok = isfinite(berr[c]) && berr[c] <= kIterTol;
+        const bool ok = isfinite(chi) && isfinite(berr[c]) && berr[c] <= kIterTol;
         if constexpr (ADJ) {          // the adjoint's z = conj(x) and the flag; no chi, no gamma
             if (h == 0) {
                 a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;

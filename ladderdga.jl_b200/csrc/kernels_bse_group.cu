@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_bse_group(const BseArgs a_m, 
         if (ql >= nvalid) continue;
         const int q = pw[ql];
         const double chi = sx / (a.beta * a.beta);
-        const bool good = isfinite(berr[mt]) && berr[mt] <= kGrpTol;
+        const bool good = isfinite(chi) && isfinite(berr[mt]) && berr[mt] <= kGrpTol;
         if (t == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = good ? 0 : 1;
