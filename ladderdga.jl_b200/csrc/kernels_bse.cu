@@ -2899,10 +2899,10 @@ struct BseVariant {
 
 #define LDGA_SMALL_BOX(N)                                                                              \
     const BseVariant fp64_##N[] = {{&run_lu<N, 8, 1, 2>, "lu8:2", &run_lu_pair<N, 8, 1, 2>},           \
-                                   {&run_lu<N, 8, 1, 4>, "lu8:4"},                                     \
-                                   {&run_lu<N, 8, 1, 8>, "lu8:8"}};                                     \
+                                   {&run_lu<N, 8, 1, 4>, "lu8:4", &run_lu_pair<N, 8, 1, 4>},           \
+                                   {&run_lu<N, 8, 1, 8>, "lu8:8", &run_lu_pair<N, 8, 1, 8>}};          \
     const BseVariant mixed_##N[] = {{&run_warp32<N, 8, 4, 4, 1>, "warp:1", &run_warp32_pair<N, 8, 4, 4, 1>}, \
-                                    {&run_warp32<N, 8, 4, 4, 3>, "warp:3"}};                           \
+                                    {&run_warp32<N, 8, 4, 4, 3>, "warp:3", &run_warp32_pair<N, 8, 4, 4, 3>}}; \
     const BseVariant inv_##N[] = {{&run_tile<N, 8, 8, 2, 1, double, LDGA_PREC_FP64_INV>, "gj8x2"}};
 LDGA_SMALL_BOX(4)
 LDGA_SMALL_BOX(6)
@@ -2917,10 +2917,10 @@ LDGA_SMALL_BOX(12)
 // groups are wide, so the autotuner decides
 #define LDGA_ITER_BOX(N, LPQ, MINB, NP, MINB_TC, TCNAME)                                                \
     const BseVariant fp64_##N[] = {{&run_lu<N, 8, 1, 2>, "lu8:2", &run_lu_pair<N, 8, 1, 2>},           \
-                                   {&run_lu<N, 8, 1, 4>, "lu8:4"},                                     \
-                                   {&run_lu<N, 8, 1, 8>, "lu8:8"}};                                     \
+                                   {&run_lu<N, 8, 1, 4>, "lu8:4", &run_lu_pair<N, 8, 1, 4>},           \
+                                   {&run_lu<N, 8, 1, 8>, "lu8:8", &run_lu_pair<N, 8, 1, 8>}};          \
     const BseVariant mixed_##N[] = {{&run_warp32<N, 8, 4, 4, 1>, "warp:1", &run_warp32_pair<N, 8, 4, 4, 1>}, \
-                                    {&run_warp32<N, 8, 4, 4, 3>, "warp:3"},                            \
+                                    {&run_warp32<N, 8, 4, 4, 3>, "warp:3", &run_warp32_pair<N, 8, 4, 4, 3>}, \
                                     {&run_iter<N, LPQ, MINB>, "iter"},                                 \
                                     {&run_iter<NP, 8, MINB_TC, 2, true, true, true, true, true, N>, TCNAME, \
                                      &run_iter_pair<NP, 8, MINB_TC, 2, true, true, true, true, true, N>}}; \
@@ -2930,8 +2930,9 @@ LDGA_ITER_BOX(20, 4, 4, 24, 4, "iter8x2dm2ns24:4")
 LDGA_ITER_BOX(30, 4, 3, 32, 3, "iter8x2dm2ns32:3")
 #undef LDGA_ITER_BOX
 constexpr int kIter30 = 3;   // the tensor-core iteration in mixed_30
-const BseVariant fp64_40[] = {{&run_lu<40, 8, 1, 6>, "lu8:6", &run_lu_pair<40, 8, 1, 6>}, {&run_lu<40, 8, 1, 4>, "lu8:4"},
-                              {&run_lu<40, 8, 1, 5>, "lu8:5"}};
+const BseVariant fp64_40[] = {{&run_lu<40, 8, 1, 6>, "lu8:6", &run_lu_pair<40, 8, 1, 6>},
+                              {&run_lu<40, 8, 1, 4>, "lu8:4", &run_lu_pair<40, 8, 1, 4>},
+                              {&run_lu<40, 8, 1, 5>, "lu8:5", &run_lu_pair<40, 8, 1, 5>}};
 // the default: the group inverse by Newton-Schulz on tcgen05 tensor cores (Gauss-Jordan as its fallback)
 const BseVariant mixed_40[] = {{&run_iter<40, 8, 3, 2, true, true, true, true, true>, "iter8x2dm2ns:3",
                                 &run_iter_pair<40, 8, 3, 2, true, true, true, true, true>},
@@ -2942,28 +2943,32 @@ const BseVariant mixed_40[] = {{&run_iter<40, 8, 3, 2, true, true, true, true, t
                                {&run_iter<40, 8, 3, 2, true, true>, "iter8x2tc:3"}, {&run_iter<40, 8, 2, 2, true, true>, "iter8x2tc:2"},
                                {&run_iter<40, 8, 2, 2>, "iter8x2:2"}, {&run_iter<40, 8, 3, 2>, "iter8x2:3"},
                                {&run_iter<40, 8, 2>, "iter8:2"}, {&run_iter<40, 4, 3>, "iter"},
-                               {&run_warp32<40, 8, 4, 4, 3>, "warp:3"}, {&run_warp32<40, 8, 4, 4, 2>, "warp:2"}};
+                               {&run_warp32<40, 8, 4, 4, 3>, "warp:3", &run_warp32_pair<40, 8, 4, 4, 3>},
+                               {&run_warp32<40, 8, 4, 4, 2>, "warp:2", &run_warp32_pair<40, 8, 4, 4, 2>}};
 const BseVariant inv_40[] = {{&run_tile<40, 8, 8, 2, 1, double, LDGA_PREC_FP64_INV>, "gj8x2"}};
-const BseVariant fp64_60[] = {{&run_lu<60, 16, 1, 2>, "lu16:2", &run_lu_pair<60, 16, 1, 2>}, {&run_lu<60, 16, 1, 1>, "lu16:1"},
-                              {&run_lu<60, 16, 1, 3>, "lu16:3"}};
+const BseVariant fp64_60[] = {{&run_lu<60, 16, 1, 2>, "lu16:2", &run_lu_pair<60, 16, 1, 2>},
+                              {&run_lu<60, 16, 1, 1>, "lu16:1", &run_lu_pair<60, 16, 1, 1>},
+                              {&run_lu<60, 16, 1, 3>, "lu16:3", &run_lu_pair<60, 16, 1, 3>}};
 // MIXED may pick any configuration whose results meet the FP64 backward-error bound, the FP64 LU
 // included: at Nν = 60 and 120 that is the fastest one measured
 // the grouped preconditioned iteration (kernels_bse_group.cu) on tiles padded to 64
 const BseVariant mixed_60[] = {{&run_group<64>, "iterg64", &run_group_pair<64>},
-                               {&run_lu<60, 16, 1, 2>, "lu16:2"}, {&run_lu32<60, 16, 1, 3>, "lu32x16:3"},
+                               {&run_lu<60, 16, 1, 2>, "lu16:2", &run_lu_pair<60, 16, 1, 2>},
+                               {&run_lu32<60, 16, 1, 3>, "lu32x16:3"},
                                {&run_lu32<60, 16, 1, 2>, "lu32x16:2"}, {&run_iter<60, 8, 1>, "iter"}};
 const BseVariant inv_60[] = {{&run_tile<60, 16, 16, 1, 1, double, LDGA_PREC_FP64_INV>, "gj16x1"}};
 // Nν = 120: Gamma(w) (230 KB) exceeds shared memory and is read through L1/L2; FP64_INV solves by LU
 // (32 x 32 threads per matrix -- a 4 x 4 register tile instead of 16 x 16 threads' spilling 8 x 8 --
 // measured 1.76x slower: 120 steps of a 1024-thread barrier over little work per thread)
-const BseVariant fp64_120[] = {{&run_lu<120, 16, 1, 1, false>, "lu16g:1"}};
+const BseVariant fp64_120[] = {{&run_lu<120, 16, 1, 1, false>, "lu16g:1", &run_lu_pair<120, 16, 1, 1, false>}};
 // MIXED at Nν = 120: the Jacobi refinement (bse_jacobi.cuh), whose stop test bounds the forward error
 // too (the test matrices' condition numbers reach 1e4, where a backward error of 1e-14 alone would
 // not guarantee the 1e-10 forward accuracy), then the LU forms
 const BseVariant mixed_120[] = {{&run_jacobi<120, 32, 4, true>, "jac", &run_jacobi_pair<120, 32, 4, true>},
                                 {&run_jacobi<120, 32, 4, false>, "jac4", &run_jacobi_pair<120, 32, 4, false>},
                                 {&run_jacobi<120, 16, 2, true>, "jac16:2", &run_jacobi_pair<120, 16, 2, true>},
-                                {&run_lu<120, 16, 1, 1, false>, "lu16g:1"}, {&run_lu32<120, 16, 1, 1, false>, "lu32x16g:1"}};
+                                {&run_lu<120, 16, 1, 1, false>, "lu16g:1", &run_lu_pair<120, 16, 1, 1, false>},
+                                {&run_lu32<120, 16, 1, 1, false>, "lu32x16g:1"}};
 
 // Box sizes without kernels of their own: the LU on the next tile up (padded), all modes; in MIXED the
 // grouped iteration above Nnu = 40, where the elimination's N^3 outgrows it.  Nnu > 112 (but 120): the
@@ -3224,9 +3229,9 @@ int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail) {
 // (channel d flags into d_flags2); the matrices it leaves above its backward-error bound are appended
 // to one list per channel (counts in d_count[2], d_count[3], zeroed by the caller with d_fail) and
 // re-solved by one pivoted launch over both lists.  Otherwise launch_bse for m, then d.  Every default
-// but FP64_INV's has the form: at the small boxes one channel alone leaves most of the chip idle and its
-// time is the chain of one matrix's elimination (Nnu = 20 on 16^2: 945 warps; the whole chain 125 us,
-// 140 us with the channels one after the other).
+// but FP64_INV's has the form, and every FP64 and warp elimination: at the small boxes one channel alone
+// leaves most of the chip idle and its time is the chain of one matrix's elimination (Nnu = 20 on 16^2: 945
+// warps; the whole chain 125 us, 140 us with the channels one after the other).
 int launch_bse_pair(ldga_ctx* ctx, int32_t* d_fail) {
     const BseVariant* v = nullptr;
     const int nv = variants_of(ctx->Nnu, ctx->prec, &v);
