@@ -664,13 +664,18 @@ def roofline(stages: dict, chain, peaks: dict, sweeps=None, steps: int = 1) -> d
             peak, peak_src = fp64_peak(peaks, sm_mhz)
             qpw = {"iter": 8, "iter8": 4, "iter8x2": 8, "iter8x2tc": 8, "iter8x2dm": 8,
                    "iter8x2dm2": 8}.get(cfg.split(":")[0], 8)
-            nprod = 2.0 if "dm2" in cfg else 1.0   # the second-order correction: two TF32 products a pass
+            grouped = cfg.startswith("iterg")
+            # TF32 products a pass: three in the third-order correction, two in the second-order one
+            nprod = 3.0 if grouped else 2.0 if "dm2" in cfg else 1.0
             passes, warps = sweeps if sweeps else (0, 1)
-            prod = 6.0 if "dm" in cfg else 8.0
+            prod = 6.0 if "dm" in cfg or grouped else 8.0
             f64 = passes * qpw * (prod * nnu**2 + 8.0 * nnu) / max(cnt, 1)
             f32 = nprod * (passes - warps) * qpw * 8.0 * nnu**2 / max(cnt, 1)
             exe = f64 / t / 1e12
-            kname = ("k_bse_iter (FP32 group inverse; FP64 residual on the FP64 tensor path, mma.sync m8n8k4, "
+            kname = ("k_bse_group (FP32 group inverse; FP64 residual on the FP64 tensor path, mma.sync m8n8k4, "
+                     "three real products per complex tile; third-order correction, three TF32 tensor-core products "
+                     "a pass; no exchange between the products)" if grouped else
+                     "k_bse_iter (FP32 group inverse; FP64 residual on the FP64 tensor path, mma.sync m8n8k4, "
                      "three real products per complex tile; second-order correction C r - C (dD C r), two TF32 "
                      "tensor-core products a pass)" if "dm2" in cfg else
                      "k_bse_iter (FP32 group inverse; FP64 residual on the FP64 tensor path, mma.sync m8n8k4, "
