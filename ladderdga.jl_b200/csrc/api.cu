@@ -168,6 +168,7 @@ int alloc_all(ldga_ctx* c) {
     TRY(dev_alloc(c, &c->d_count, 4));
     TRY(dev_alloc(c, &c->d_qperm, nq * nw));
     TRY(dev_alloc(c, &c->d_iter_stats, 2));
+    TRY(grow_buffer(c, &c->d_partial, &c->partial_elems, eom_partial_need(c)));
     LDGA_CUDA(c, cudaMemset(c->d_iter_stats, 0, 2 * sizeof(unsigned long long)));
     if (bse_pivot_smem((int)nnu) > LDGA_PIVOT_SMEM_MAX)
         TRY(dev_alloc(c, &c->d_pivot_scratch, (size_t)LDGA_PIVOT_GRID * nnu * (nnu + 1)));
@@ -316,11 +317,7 @@ int set_sigma_loc(ldga_ctx* ctx, const double* sigma_loc, int n_sigma) {
     if (n_sigma <= L)
         return ctx_fail(ctx, LDGA_ERR_ARG, "Sigma_loc must cover n = 0..max|fft_range| (" + std::to_string(L + 1) +
                                                " values), got " + std::to_string(n_sigma));
-    if (n_sigma > ctx->n_sigma_loc) {
-        if (ctx->d_sigma_loc) cudaFree(ctx->d_sigma_loc);
-        ctx->d_sigma_loc = nullptr;
-        TRY(dev_alloc(ctx, &ctx->d_sigma_loc, (size_t)n_sigma));
-    }
+    TRY(grow_buffer(ctx, &ctx->d_sigma_loc, &ctx->n_sigma_alloc, (size_t)n_sigma));
     ctx->n_sigma_loc = n_sigma;
     return copy(ctx, ctx->d_sigma_loc, sigma_loc, (size_t)n_sigma * sizeof(double2));
 }
@@ -1235,20 +1232,10 @@ int chain_m_submit(ldga_ctx* ctx, const ChainArgs& a, bool use_graph, bool* repl
     const int need_g = 2 * ctx->sp.n_iv + ctx->sp.n_iw + (ctx->sp.shift ? ctx->sp.n_iw : 0);
     if (n_gimp < need_g) return ctx_fail(ctx, LDGA_ERR_ARG, "G_imp too short for the frequency box");
     // buffers (allocated outside any capture)
-    if (n_sigma > ctx->n_sigma_loc) {
-        if (ctx->d_sigma_loc) cudaFree(ctx->d_sigma_loc);
-        ctx->d_sigma_loc = nullptr;
-        TRY(dev_alloc(ctx, &ctx->d_sigma_loc, (size_t)n_sigma));
-        ctx->n_sigma_loc = n_sigma;
-    }
+    TRY(grow_buffer(ctx, &ctx->d_sigma_loc, &ctx->n_sigma_alloc, (size_t)n_sigma));
     ctx->n_sigma_loc = std::max(ctx->n_sigma_loc, (int)n_sigma);
     TRY(dev_alloc(ctx, &ctx->d_chiloc, (size_t)ctx->Nnu * ctx->Nnu * ctx->Nw));
-    if (n_gimp > ctx->n_gimp_alloc) {
-        if (ctx->d_gimp) cudaFree(ctx->d_gimp);
-        ctx->d_gimp = nullptr;
-        TRY(dev_alloc(ctx, &ctx->d_gimp, (size_t)n_gimp));
-        ctx->n_gimp_alloc = n_gimp;
-    }
+    TRY(grow_buffer(ctx, &ctx->d_gimp, &ctx->n_gimp_alloc, (size_t)n_gimp));
     if (!ctx->h_stage) LDGA_CUDA(ctx, cudaMallocHost(reinterpret_cast<void**>(&ctx->h_stage), 64 * sizeof(double) + 16));
     if (!ctx->io_stream) {
         LDGA_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->io_stream, cudaStreamNonBlocking));
@@ -1267,7 +1254,7 @@ int chain_m_submit(ldga_ctx* ctx, const ChainArgs& a, bool use_graph, bool* repl
                                dbits(ctx->mp.U), dbits(ctx->mp.mu), dbits(ctx->mp.beta), dbits(ctx->mp.n),
                                dbits(ctx->mp.Ekin_DMFT), (uint64_t)ctx->prec, (uint64_t)(uintptr_t)ctx->stream,
                                (uint64_t)ctx->profiling, (uint64_t)ctx->prof_mask, (uint64_t)ctx->newton_cluster,
-                               (uint64_t)ctx->l0_beside});
+                               (uint64_t)ctx->l0_beside, ctx->buf_gen});
     }
     if (graphable && ctx->graph_exec && key == ctx->graph_key) {
         LDGA_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, ctx->stream));
@@ -1438,10 +1425,8 @@ int dm_lanes_ready(ldga_ctx* ctx) {
     const size_t nsig = (size_t)ctx->Nq * std::max(ctx->Nnu, 1);
     for (int j = 0; j < 2; ++j) {
         LDGA_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->dm_sigma[j]), nsig * sizeof(double2)));
-        if (ctx->partial_elems) {
-            LDGA_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->dm_partial[j]), ctx->partial_elems * sizeof(double2)));
-            ctx->dm_partial_elems[j] = ctx->partial_elems;
-        }
+        LDGA_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->dm_partial[j]), ctx->partial_elems * sizeof(double2)));
+        ctx->dm_partial_elems[j] = ctx->partial_elems;
     }
     return LDGA_OK;
 }

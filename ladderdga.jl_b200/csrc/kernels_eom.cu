@@ -117,12 +117,13 @@ __global__ void __launch_bounds__((kThrOne<DIM, N, TC>), 1) k_eom_inverse(
 // vectors costs about 1 + np / 2 whatever np is, and the launch takes the rounds its CTAs need on the
 // SMs' slots times the steps of one CTA (3D 32^3, 20 ν x 41 ω: 2 ω per CTA in 1.4 rounds 48 us, 3 ω
 // in one round 41 us; 2D 64^2, 22 ν x 61 ω: 2 ω 36 us, 5 ω 30 us).
-struct EomShape { int wpc, np; };
+// The split is not monotone in numax: fewer ν can need more partial sums (2D 64^2, 61 ω: 270 rows at
+// 30 ν, 589 at 19), so the handle's buffer is sized for every numax at once (eom_partial_need).
 template <int DIM, int N>
 EomShape eom_shape(int numax, int nw, bool tc) {
     using P = TransformPlan<DIM, N>;
     const int npm = tc ? std::max(1, std::min(16, (int)(kSmemBudgetTC / P::SMEM1))) : P::NP;
-    EomShape best{1, 1};
+    EomShape best;
     double bt = 1e300;
     for (int np = 1; np <= npm; ++np) {
         const int by_smem = (int)((size_t)227 * 1024 / (np * P::SMEM1 + P::S::NQ * sizeof(double2) + 2048));
@@ -136,20 +137,38 @@ EomShape eom_shape(int numax, int nw, bool tc) {
     return best;
 }
 
+// eom_shape, computed once per numax and number of ω (the search takes 1.5 to 6.5 us)
+template <int DIM, int N>
+EomShape eom_shape_of(ldga_ctx* ctx, int numax, int nw) {
+    if (ctx->eom_shapes_nw != nw || (int)ctx->eom_shapes.size() < numax) {
+        ctx->eom_shapes.assign(std::max(numax, ctx->Nnu), EomShape{});
+        ctx->eom_shapes_nw = nw;
+    }
+    EomShape& s = ctx->eom_shapes[numax - 1];
+    if (s.np == 0) s = eom_shape<DIM, N>(numax, nw, ctx->transform_tc);
+    return s;
+}
+
+template <int DIM, int N>
+size_t partial_need(ldga_ctx* ctx) {
+    size_t need = 0;
+    for (int numax = 1; numax <= ctx->Nnu; ++numax) {
+        const int wpc = eom_shape_of<DIM, N>(ctx, numax, ctx->Nw).wpc;
+        need = std::max(need, (size_t)((ctx->Nw + wpc - 1) / wpc) * numax * ctx->Nq);
+    }
+    return need;
+}
+
 template <int DIM, int N>
 int run_eom(ldga_ctx* ctx, int numax, double lam_m, double lam_d, const double* lm_dev, const double* ld_dev,
             int part, int& nchunk_out) {
     const int nws = shard_nw(ctx);
-    const EomShape shape = eom_shape<DIM, N>(numax, nws, ctx->transform_tc);
+    const EomShape shape = eom_shape_of<DIM, N>(ctx, numax, nws);
     const int wpc = shape.wpc, np = shape.np;
     const int nchunk = (nws + wpc - 1) / wpc;
-    const size_t need = (size_t)nchunk * numax * ctx->Nq;
-    if (need > ctx->partial_elems) {
-        if (ctx->d_partial) cudaFree(ctx->d_partial);
-        ctx->d_partial = nullptr;
-        LDGA_CUDA(ctx, cudaMalloc(&ctx->d_partial, need * sizeof(double2)));
-        ctx->partial_elems = need;
-    }
+    // allocated with the handle; only an ω shard can need more
+    const int gs = grow_buffer(ctx, &ctx->d_partial, &ctx->partial_elems, (size_t)nchunk * numax * ctx->Nq);
+    if (gs != LDGA_OK) return gs;
     EomArgs a;
     a.nnu = ctx->Nnu; a.nw = ctx->Nw; a.n_iv = ctx->sp.n_iv; a.n_iw = ctx->sp.n_iw; a.shift = ctx->sp.shift;
     a.fft_lo = ctx->fft_lo; a.numax = numax; a.w_per_chunk = wpc;
@@ -194,6 +213,13 @@ int run_eom_all(ldga_ctx* ctx, int numax, double lam_m, double lam_d, const doub
     return run_eom_inverse<DIM, N>(ctx, numax, nchunk, d_tail, tc, chiloc_m_sum, out, out_ld, add_hartree);
 }
 }  // namespace
+
+size_t eom_partial_need(ldga_ctx* ctx) {
+#define BODY(D, NS) partial_need<D, NS>(ctx)
+    LDGA_FOR_EACH_GRID(LDGA_CASE)
+#undef BODY
+    return 0;
+}
 
 int launch_eom(ldga_ctx* ctx, int numax, double lam_m, double lam_d, const double* lam_m_dev,
                const double* lam_d_dev, int part, const double* d_tail, int tc, double chiloc_m_sum,

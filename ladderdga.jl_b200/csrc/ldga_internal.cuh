@@ -71,6 +71,9 @@ struct TMat {
 // ------------------------------------------------------------------------------------------
 // handle
 // ------------------------------------------------------------------------------------------
+// the EoM forward kernel's split: ω per CTA, vectors per step (np = 0: not computed yet)
+struct EomShape { int wpc = 0, np = 0; };
+
 struct ldga_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -89,7 +92,7 @@ struct ldga_ctx {
     double2* d_ghat = nullptr;     // [Nq, Nf]   transformed G, R on the wedge
     double2* d_gloc = nullptr;     // [Nq, Nf]   G(k, nu)
     double2* d_sigma_loc = nullptr;
-    int n_sigma_loc = 0;
+    int n_sigma_loc = 0, n_sigma_alloc = 0;   // values set, values the buffer holds
     double2* d_chi0 = nullptr;     // [Nq, Nnu, Nw]
     double2* d_Gamma[2] = {nullptr, nullptr};   // [Nnu, Nnu, Nw]
     double* d_chi[2] = {nullptr, nullptr};      // [Nq, Nw]
@@ -101,6 +104,8 @@ struct ldga_ctx {
     double2* d_gladder = nullptr;  // [Nq, Nf]
     double2* d_partial = nullptr;  // EoM partial sums [nchunk, Nq, numax]
     size_t partial_elems = 0;
+    std::vector<EomShape> eom_shapes;   // [numax - 1], for eom_shapes_nw bosonic frequencies
+    int eom_shapes_nw = 0;
     double* d_red = nullptr;       // reduction scratch
     int32_t* d_flags = nullptr;    // BSE fallback flags [Nq*Nw]
     int32_t* d_flags2 = nullptr;   // the d channel's flags when both channels run in one launch
@@ -152,6 +157,9 @@ struct ldga_ctx {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     std::vector<uint64_t> graph_key;
+    // part of the key: counts the buffers of the chain that were replaced by larger ones (d_partial,
+    // d_sigma_loc, d_gimp), whose addresses a captured graph holds
+    uint64_t buf_gen = 0;
     std::vector<std::pair<int, int>> graph_ev;   // stage events recorded inside the captured graph
     int64_t graph_launches = 0;                  // kernels per replay of the captured graph
     double* h_stage = nullptr;     // pinned host staging for the chain's scalars (64 doubles + 4 ints)
@@ -201,6 +209,22 @@ int ctx_cuda(ldga_ctx* ctx, cudaError_t e, const char* what);
         cudaError_t _e = cudaGetLastError();                        \
         if (_e != cudaSuccess) return ctx_cuda((ctx), _e, what);    \
     } while (0)
+
+// A buffer of at least n elements: replaced by a larger one (its contents are not kept) when it has fewer.
+// The old one is freed after the allocation, so a failure leaves the handle as it was; a graph captured
+// with the old address is not replayed any more (buf_gen).
+template <typename T, typename N>
+inline int grow_buffer(ldga_ctx* ctx, T** p, N* have, size_t n) {
+    if (*p && n <= (size_t)*have) return LDGA_OK;
+    if (ctx->capturing) return ctx_fail(ctx, LDGA_ERR_STATE, "buffer too small under capture");
+    T* fresh = nullptr;
+    LDGA_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&fresh), (n > 0 ? n : 1) * sizeof(T)));
+    if (*p) cudaFree(*p);
+    *p = fresh;
+    *have = (N)n;
+    ctx->buf_gen++;
+    return LDGA_OK;
+}
 
 // Dynamic shared-memory opt-in for a kernel; skipped while a CUDA graph is being captured (the
 // uncaptured warm-up run of the same sequence has already set it).
@@ -272,6 +296,8 @@ int launch_lambda0(ldga_ctx* ctx);
 int launch_lambda0_vjp(ldga_ctx* ctx, const double2* l0_bar, double2* chi0_bar);
 // dE_pot,1/dΣ_ladder [Nq, numax] with μ following the filling condition (calc_E after G_from_Σladder!)
 int launch_epot_vjp(ldga_ctx* ctx, int numax, double mu, const double2* sigma, double2* out);
+// Elements of the EoM's partial sums that hold every numax of the handle's box at the whole ω range
+size_t eom_partial_need(ldga_ctx* ctx);
 // EoM forward + inverse.  lam_*_dev (may be null) are device scalars added to lam_m / lam_d.
 int launch_eom(ldga_ctx* ctx, int numax, double lam_m, double lam_d, const double* lam_m_dev,
                const double* lam_d_dev, int part, const double* d_tail, int tc, double chiloc_m_sum,
