@@ -170,8 +170,8 @@ int ldga_bse(ldga_ctx* ctx, int32_t channel, const double* gamma_r_in, double* c
  * gamma_r [Nq, Nnu, Nw] (complex, dL/dRe + i dL/dIm), either may be NULL for zero, returns
  *   Gamma_bar [Nnu, Nnu, Nw] = dL/dGamma_r   and   chi0_bar [Nq, Nnu, Nw] = dL/dchi0
  * in the same convention (either output may be NULL).  One FP64 adjoint solve per (q, w) with the
- * untransposed vertex, verified by its backward error; n_flagged (may be NULL) counts solves
- * above 1e-12.  The forward solution is rebuilt from gamma_r and chi_r, not recomputed. */
+ * untransposed vertex, verified by its backward error; a solve above 1e-12 or with a non-finite solution
+ * is repeated with partial pivoting, and n_flagged (may be NULL) counts those that stay non-finite.  The forward solution is rebuilt from gamma_r and chi_r, not recomputed. */
 int ldga_bse_vjp(ldga_ctx* ctx, int32_t channel, const double* chi_bar, const double* gam_bar,
                  double* Gamma_bar, double* chi0_bar, int32_t* n_flagged);
 
@@ -205,7 +205,7 @@ int ldga_gloc_vjp(ldga_ctx* ctx, const double* chi0_bar, const double* lambda0_b
  * handle's current chi, gamma, lambda_0 (e.g. right after ldga_chain_m).  Outputs (any may be NULL):
  * Gamma_m_bar, Gamma_d_bar [Nnu, Nnu, Nw], sigma_loc_bar [n_sigma] = dL/dSigma_loc(nu_n) through the
  * lattice G, chi0_bar [Nq, Nnu, Nw] = the total dL/dchi0.  Pointers may be host or device memory.
- * n_flagged (may be NULL): adjoint solves of both channels above the backward-error threshold. */
+ * n_flagged (may be NULL): adjoint solves of both channels that stay non-finite with partial pivoting. */
 int ldga_chain_vjp(ldga_ctx* ctx, const double* sigma_bar, double lam_m, double lam_d, int32_t numax, int32_t tc,
                    double* Gamma_m_bar, double* Gamma_d_bar, int32_t n_sigma, double* sigma_loc_bar,
                    double* chi0_bar, int32_t* n_flagged);

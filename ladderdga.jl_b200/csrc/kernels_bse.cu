@@ -2299,7 +2299,8 @@ __global__ void __launch_bounds__(kIterQ * LPQ / QPL, MINB) k_bse_iter(const Bse
 //   chi_bar_tot = chi_bar - s U rf^2 sum_i Re(conj(gamma_bar_i) y_i d_i)
 //   y_bar_i = conj(d_i rf) gamma_bar_i + chi_bar_tot / beta^2
 //   z = B^-H y_bar  <=>  (Gamma(w) + diag(d)) conj(z) = conj(y_bar): the same LU kernel on the
-//       untransposed vertex (one FP64 solve per matrix, verified by its backward error)
+//       untransposed vertex (one FP64 solve per matrix, verified by its backward error; a matrix above
+//       1e-12 or with a non-finite solution is solved again with partial pivoting, k_bse_adj_pivot)
 //   B_bar = -z y^H  ->  Gamma_bar(w)[a, b] = -sum_q conj(y_a) z_b  (k_bse_gamma_grad)
 //   chi0_bar_i = -conj(d_i^2) (conj(y_i rf) gamma_bar_i - z_i conj(y_i))
 // This is the chi-bar contraction of the inverse, chi^T chi_bar chi^T, restricted to the single
@@ -2318,9 +2319,11 @@ struct BseAdjArgs {
     int accumulate;
     double2* ybuf;            // [Nq, N, Nw]   out: y
     double2* zbuf;            // [Nq, N, Nw]   out: z
-    int32_t* flags;           // [Nq, Nw]      1: backward error above 1e-12
-    const int32_t* list = nullptr;    // k_bse_adj: only these (q + Nq w), count[0] of them
+    int32_t* flags;           // [Nq, Nw]      1: left to the next solve
+    const int32_t* list = nullptr;    // only these (q + Nq w), count[0] of them (null: k_bse_adj takes all)
     const int32_t* count = nullptr;
+    int32_t* fail_list = nullptr;     // k_bse_adj: what it leaves to k_bse_adj_pivot, at atomicAdd(fail_count)
+    int32_t* fail_count = nullptr;
 };
 
 template <int N, int T, int MINB>
@@ -2463,9 +2466,9 @@ __global__ void __launch_bounds__(T * T, MINB) k_bse_adj(const BseAdjArgs a) {
                 for (int ra = 0; ra < r; ++ra) acc[ra] = cadd(acc[ra], cmul(b[ra][r], xj));
             }
         }
-        // ---- FP64 backward error |rhs - A x| / (|A| |x| + |rhs|)
-        double st[4] = {0.0, 0.0, 0.0, 0.0};
-        const int op[4] = {1, 1, 1, 1};
+        // ---- FP64 backward error |rhs - A x| / (|A| |x| + |rhs|), and the sum of x: the maxima drop a NaN
+        double st[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        const int op[5] = {1, 1, 1, 1, 0};
 #pragma unroll
         for (int ra = 0; ra < RT; ++ra) {
             const int i = tr + T * ra;
@@ -2495,20 +2498,26 @@ __global__ void __launch_bounds__(T * T, MINB) k_bse_adj(const BseAdjArgs a) {
                 st[1] = fmax(st[1], fabs(xv.x) + fabs(xv.y));
                 st[2] = fmax(st[2], rown);
                 st[3] = fmax(st[3], fabs(rhs[i].x) + fabs(rhs[i].y));
+                st[4] += xv.x + xv.y;
             }
         }
-        group_reduce<4, G>(st, op, red, bar, t);
+        group_reduce<5, G>(st, op, red, bar, t);
         const double berr = st[0] / (st[2] * st[1] + st[3] + 1e-300);
-        if (t == 0) a.flags[cq] = (isfinite(berr) && berr <= 1e-12) ? 0 : 1;
+        const bool ok = isfinite(st[4]) && isfinite(berr) && berr <= 1e-12;
+        if (t == 0) {
+            a.flags[cq] = ok ? 0 : 1;
+            if (!ok) a.fail_list[atomicAdd(a.fail_count, 1)] = (int32_t)cq;
+        }
         // ---- z = conj(x); chi0_bar; y and z for the vertex gradient
         for (int i = t; i < N; i += G) {
             const size_t ci = (size_t)q + (size_t)a.nq * (i + (size_t)N * w);
             const double2 z = cconj(xsm[i]), y = yfw[i], d = dinv[i];
+            a.ybuf[ci] = y;
+            if (!ok) continue;
             double2 db = cscale(cmul(z, cconj(y)), -1.0);                        // from B
             if (a.gam_bar) db = cadd(db, cmul(cconj(cscale(y, rf)), a.gam_bar[ci]));   // from gamma
             const double2 c0b = cscale(cmul(cconj(cmul(d, d)), db), -1.0);
             a.chi0_bar[ci] = a.accumulate ? cadd(a.chi0_bar[ci], c0b) : c0b;
-            a.ybuf[ci] = y;
             a.zbuf[ci] = z;
         }
         named_barrier(bar, G);
@@ -2639,22 +2648,10 @@ __device__ __forceinline__ double block_sum_det(double v, double* red) {
 // matrices and for box sizes without a tiled instantiation.  list == nullptr: all (q, w);
 // count_dev (may be null) holds the number of list entries (written earlier on the stream).
 // gscratch (may be null): LDGA_PIVOT_GRID matrices in HBM, used when [N][N+1] exceeds shared memory.
-// One flagged matrix lin = q + Nq w: the pivoted FP64 LU of [B | 1] in B (the CTA's [N][N+1] scratch);
-// writes chi, gamma and the flag (0 solved, 2 non-finite); returns true when chi is finite.  Every
-// thread of the CTA calls it.
-__device__ bool pivot_solve(const BseArgs& a, int lin, double2* B, double* red, int* piv_s) {
-    const int N = a.nnu;
+// Partial-pivoting FP64 LU of [B | rhs] in B ([N][N+1] row-major, rhs last) and the back substitution: the
+// solution takes the place of rhs.  Every thread of the CTA calls it, with B published by a barrier.
+__device__ void pivot_lu(int N, double2* B, double* red, int* piv_s) {
     const int ld = N + 1;
-    const int q = lin % a.nq, w = lin / a.nq;
-    const double2* Gw = a.Gamma + (size_t)w * N * N;
-    for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
-        const int ii = e / N, j = e - ii * N;
-        double2 g = Gw[(size_t)ii * N + j];       // Gamma[j, ii] -> B[ii][j]
-        if (ii == j) g = cadd(g, cinv(a.chi0[(size_t)q + (size_t)a.nq * (ii + (size_t)N * w)]));
-        B[ii * ld + j] = g;
-    }
-    for (int ii = threadIdx.x; ii < N; ii += blockDim.x) B[ii * ld + N] = dmk(1.0, 0.0);
-    __syncthreads();
     for (int k = 0; k < N; ++k) {
         // pivot search (cabs1, as izamax) by warp 0
         if (threadIdx.x < 32) {
@@ -2699,6 +2696,25 @@ __device__ bool pivot_solve(const BseArgs& a, int lin, double2* B, double* red, 
         if (threadIdx.x == 0) B[k * ld + N] = cdiv(csub(B[k * ld + N], dmk(re, im)), B[k * ld + k]);
         __syncthreads();
     }
+}
+
+// One flagged matrix lin = q + Nq w: the pivoted FP64 LU of [B | 1] in B (the CTA's [N][N+1] scratch);
+// writes chi, gamma and the flag (0 solved, 2 non-finite); returns true when chi is finite.  Every
+// thread of the CTA calls it.
+__device__ bool pivot_solve(const BseArgs& a, int lin, double2* B, double* red, int* piv_s) {
+    const int N = a.nnu;
+    const int ld = N + 1;
+    const int q = lin % a.nq, w = lin / a.nq;
+    const double2* Gw = a.Gamma + (size_t)w * N * N;
+    for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
+        const int ii = e / N, j = e - ii * N;
+        double2 g = Gw[(size_t)ii * N + j];       // Gamma[j, ii] -> B[ii][j]
+        if (ii == j) g = cadd(g, cinv(a.chi0[(size_t)q + (size_t)a.nq * (ii + (size_t)N * w)]));
+        B[ii * ld + j] = g;
+    }
+    for (int ii = threadIdx.x; ii < N; ii += blockDim.x) B[ii * ld + N] = dmk(1.0, 0.0);
+    __syncthreads();
+    pivot_lu(N, B, red, piv_s);
     double ys = 0.0;
     for (int ii = threadIdx.x; ii < N; ii += blockDim.x) ys += B[ii * ld + N].x;
     const double chi = block_sum_det(ys, red) / (a.beta * a.beta);
@@ -2751,9 +2767,61 @@ __global__ void __launch_bounds__(256) k_bse_lu_pivot_pair(const BseArgs am, con
     }
 }
 
-__global__ void k_count_flags(const int32_t* flags, int n, int32_t* count) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
-        if (flags[e] != 0) atomicAdd(count, 1);
+// The adjoint solves k_bse_adj left (a.list), with partial pivoting, from the y it wrote; a solution that stays
+// non-finite adds one to *d_fail.  One matrix per CTA; the list is empty on well-conditioned inputs, where
+// the launch takes the place of a count over the flags.
+__global__ void __launch_bounds__(256) k_bse_adj_pivot(const BseAdjArgs a, int32_t* d_fail) {
+    extern __shared__ double2 sm[];
+    const int N = a.nnu, ld = N + 1;
+    double* red = reinterpret_cast<double*>(sm);
+    int* piv_s = reinterpret_cast<int*>(red + 64);
+    double2* B = reinterpret_cast<double2*>(piv_s + 4);
+    const int n = min(max(a.count[0], 0), a.nq * a.nw);
+    for (int item = blockIdx.x; item < n; item += gridDim.x) {
+        const int lin = a.list[item], q = lin % a.nq, w = lin / a.nq;
+        const size_t c0 = (size_t)q + (size_t)a.nq * ((size_t)N * w);      // (q, 0, w)
+        const double rf = 1.0 / (1.0 + a.s * a.U * a.chi[lin]);
+        double s1 = 0.0;
+        if (a.gam_bar)
+            for (int i = threadIdx.x; i < N; i += blockDim.x) {
+                const size_t ci = c0 + (size_t)a.nq * i;
+                const double2 gb = a.gam_bar[ci], yd = cmul(a.ybuf[ci], cinv(a.chi0[ci]));
+                s1 += gb.x * yd.x + gb.y * yd.y;
+            }
+        s1 = block_sum_det(s1, red);
+        const double xbar = (a.chi_bar ? a.chi_bar[lin] : 0.0) - a.s * a.U * rf * rf * s1;
+        const double2* Gw = a.Gamma + (size_t)w * N * N;
+        for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
+            const int j = e / N, i = e - j * N;                            // Gamma[i, j]
+            const double2 g = Gw[e];
+            B[i * ld + j] = i == j ? cadd(g, cinv(a.chi0[c0 + (size_t)a.nq * i])) : g;
+        }
+        for (int i = threadIdx.x; i < N; i += blockDim.x) {
+            const size_t ci = c0 + (size_t)a.nq * i;
+            double2 yb = dmk(xbar / (a.beta * a.beta), 0.0);
+            if (a.gam_bar) yb = cadd(yb, cmul(cconj(cscale(cinv(a.chi0[ci]), rf)), a.gam_bar[ci]));
+            B[i * ld + N] = cconj(yb);
+        }
+        __syncthreads();
+        pivot_lu(N, B, red, piv_s);
+        double sum = 0.0;
+        for (int i = threadIdx.x; i < N; i += blockDim.x) {
+            const size_t ci = c0 + (size_t)a.nq * i;
+            const double2 z = cconj(B[i * ld + N]), y = a.ybuf[ci], d = cinv(a.chi0[ci]);
+            double2 db = cscale(cmul(z, cconj(y)), -1.0);
+            if (a.gam_bar) db = cadd(db, cmul(cconj(cscale(y, rf)), a.gam_bar[ci]));
+            const double2 c0b = cscale(cmul(cconj(cmul(d, d)), db), -1.0);
+            a.chi0_bar[ci] = a.accumulate ? cadd(a.chi0_bar[ci], c0b) : c0b;
+            a.zbuf[ci] = z;
+            sum += z.x + z.y;
+        }
+        sum = block_sum_det(sum, red);
+        if (threadIdx.x == 0) {
+            a.flags[lin] = isfinite(sum) ? 0 : 2;
+            if (!isfinite(sum)) atomicAdd(d_fail, 1);
+        }
+        __syncthreads();
+    }
 }
 
 template <int N, int TR, int TC, int MPC, int MINB, typename TF, int MODE>
@@ -3063,7 +3131,8 @@ BseArgs bse_args(ldga_ctx* ctx, int channel) {
 // The same formulas as k_bse_adj, split around the solve:
 //   k_adj_rhs:     y = gamma chi0 / rf -> ybuf; conj(y_bar) -> zbuf (the right-hand side)
 //   k_bse_iter:    zbuf <- z = conj(x) for the solved matrices, flags 1 for the others
-//   k_adj_chi0bar: chi0_bar from y, z for the unflagged matrices (k_bse_adj writes the others)
+//   k_adj_chi0bar: chi0_bar from y, z for the unflagged matrices (k_bse_adj, or k_bse_adj_pivot, writes
+//                  the others)
 
 // dst[w][i N + j] = src[w][j N + i]
 __global__ void k_transpose_gamma(int n, int nw, const double2* __restrict__ src, double2* __restrict__ dst) {
@@ -3280,6 +3349,11 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
     a.chi0_bar = chi0_bar; a.ybuf = ybuf; a.zbuf = zbuf;
     a.accumulate = accumulate ? 1 : 0;
     a.flags = ctx->d_flags;
+    if (!ctx->d_list2)
+        LDGA_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->d_list2), (size_t)ctx->Nq * ctx->Nw * sizeof(int32_t)));
+    a.fail_list = ctx->d_list2;
+    a.fail_count = ctx->d_count + 3;
+    LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count + 2, 0, 2 * sizeof(int32_t), ctx->stream));   // both lists
     int st = LDGA_OK;
     if (ctx->prec == LDGA_PREC_MIXED && ctx->Nnu == 40) {
         // MIXED: the preconditioned iteration on the transposed systems, the LU for what it leaves
@@ -3301,7 +3375,6 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
         b.stats = nullptr;
         b.fail_list = ctx->d_list;
         b.fail_count = ctx->d_count + 2;
-        LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count + 2, 0, sizeof(int32_t), ctx->stream));
         st = run_iter_impl<N, 8, 2, 2, true, true, true, true, true, N, true>(ctx, b, nullptr);
         if (st != LDGA_OK) return st;
         // chi0_bar of the solved matrices first: the LU below clears the flags of those it solves
@@ -3332,11 +3405,13 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
     }
     }
     if (st != LDGA_OK) return st;
-    st = launch_gamma_grad(ctx, ybuf, zbuf, gamma_bar);
-    if (st != LDGA_OK) return st;
-    k_count_flags<<<148, 256, 0, ctx->stream>>>(ctx->d_flags, ctx->Nq * ctx->Nw, d_fail);
-    LDGA_LAUNCHED(ctx, "k_count_flags");
-    return LDGA_OK;
+    a.list = ctx->d_list2;
+    a.count = ctx->d_count + 3;
+    const size_t smp = bse_pivot_smem(ctx->Nnu);      // at most 60 rows: 60 KB
+    LDGA_CUDA(ctx, set_smem(ctx, k_bse_adj_pivot, smp));
+    k_bse_adj_pivot<<<LDGA_PIVOT_GRID, 256, smp, ctx->stream>>>(a, d_fail);
+    LDGA_LAUNCHED(ctx, "k_bse_adj_pivot");
+    return launch_gamma_grad(ctx, ybuf, zbuf, gamma_bar);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -272,8 +272,8 @@ int launch_bubble(ldga_ctx* ctx);
 int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail);
 int launch_bse_pair(ldga_ctx* ctx, int32_t* d_fail);
 // Adjoint of one BSE channel: chi0_bar (written, or added to when accumulate), y and z buffers
-// [Nq, Nnu, Nw], Gamma_bar [Nnu, Nnu, Nw]; the number of adjoint solves above the backward-error
-// threshold is added to d_fail.
+// [Nq, Nnu, Nw], Gamma_bar [Nnu, Nnu, Nw]; the number of adjoint solves that stay non-finite with partial
+// pivoting is added to d_fail.
 int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const double2* gam_bar, double2* chi0_bar,
                    double2* ybuf, double2* zbuf, double2* gamma_bar, int32_t* d_fail, bool accumulate = false);
 // Adjoint of the EoM at (lam_m, lam_d): sbar [numax][Nq] -> gm_bar, gd_bar, l0_bar [Nq, Nnu, Nw] (pre-zeroed;
