@@ -25,6 +25,6 @@ struct BseArgs {
 
 // q order of the preconditioned solves (k_bse_qorder), computed once per chi0; nnu: the box size
 int bse_ensure_qorder(ldga_ctx* ctx, const BseArgs& a, int nnu);
-// The grouped preconditioned iteration (kernels_bse_group.cu) on tiles of `tile` rows (a multiple of 8,
-// 16..64, at least nnu and less than nnu + 8); ad: the second channel in the same launch, or null.
-int run_bse_group(ldga_ctx* ctx, int tile, const BseArgs& a, const BseArgs* ad);
+// The grouped preconditioned iteration (kernels_bse_group.cu) on tiles of 64 rows (boxes of 57..64); ad: the
+// second channel in the same launch, or null.
+int run_bse_group(ldga_ctx* ctx, const BseArgs& a, const BseArgs* ad);

@@ -24,7 +24,7 @@
 //                       y = row sums of B^-1.
 //   LDGA_PREC_FP64      FP64 elimination of [B | 1].
 //   LDGA_PREC_MIXED     per box size the fastest of: the q-shared preconditioned iteration
-//                       (k_bse_iter, and k_bse_group of kernels_bse_group.cu for Nν = 42 .. 64: an FP32
+//                       (k_bse_iter, and k_bse_group of kernels_bse_group.cu at Nν = 60: an FP32
 //                       inverse per group of q, FP64 residual sweeps; at
 //                       Nν = 40 both products on tensor cores: FP64 mma.sync m8n8k4 for the residual,
 //                       TF32 m16n8k8 for the correction), an FP32 elimination with FP64
@@ -2950,14 +2950,8 @@ int run_iter_pair(ldga_ctx* ctx, const BseArgs& a_m, const BseArgs& a_d) {
     return run_iter_impl<N, LPQ, MINB, QPL, GSM, TC, DM, P2, NS, NL>(ctx, a_m, &a_d);
 }
 
-template <int TILE>
-int run_group(ldga_ctx* ctx, const BseArgs& a) {
-    return run_bse_group(ctx, TILE, a, nullptr);
-}
-template <int TILE>
-int run_group_pair(ldga_ctx* ctx, const BseArgs& a_m, const BseArgs& a_d) {
-    return run_bse_group(ctx, TILE, a_m, &a_d);
-}
+int run_group(ldga_ctx* ctx, const BseArgs& a) { return run_bse_group(ctx, a, nullptr); }
+int run_group_pair(ldga_ctx* ctx, const BseArgs& a_m, const BseArgs& a_d) { return run_bse_group(ctx, a_m, &a_d); }
 
 struct BseVariant {
     BseRun run;
@@ -3020,7 +3014,7 @@ const BseVariant fp64_60[] = {{&run_lu<60, 16, 1, 2>, "lu16:2", &run_lu_pair<60,
 // MIXED may pick any configuration whose results meet the FP64 backward-error bound, the FP64 LU
 // included: at Nν = 60 and 120 that is the fastest one measured
 // the grouped preconditioned iteration (kernels_bse_group.cu) on tiles padded to 64
-const BseVariant mixed_60[] = {{&run_group<64>, "iterg64", &run_group_pair<64>},
+const BseVariant mixed_60[] = {{&run_group, "iterg64", &run_group_pair},
                                {&run_lu<60, 16, 1, 2>, "lu16:2", &run_lu_pair<60, 16, 1, 2>},
                                {&run_lu32<60, 16, 1, 3>, "lu32x16:3"},
                                {&run_lu32<60, 16, 1, 2>, "lu32x16:2"}, {&run_iter<60, 8, 1>, "iter"}};
@@ -3038,9 +3032,11 @@ const BseVariant mixed_120[] = {{&run_jacobi<120, 32, 4, true>, "jac", &run_jaco
                                 {&run_lu<120, 16, 1, 1, false>, "lu16g:1", &run_lu_pair<120, 16, 1, 1, false>},
                                 {&run_lu32<120, 16, 1, 1, false>, "lu32x16g:1"}};
 
-// Box sizes without kernels of their own: the LU on the next tile up (padded), all modes; in MIXED the
-// grouped iteration above Nnu = 40, where the elimination's N^3 outgrows it.  Nnu > 112 (but 120): the
-// pivoted kernel (a 128 x 129 register tile spills, Gamma(w) outgrows shared memory).
+// Box sizes without kernels of their own: the FP64 LU on the next tile up (padded), in every mode.  (MIXED on the
+// grouped iteration at 42..64 was no faster below 100 q and 50 to 4000 times further from the exact solution than
+// the FP64 elimination: 45 q x 25 w, Nnu = 46 202 us a call against 149, errors of chi 2.5e-14 to 4e-13
+// against 3e-16.)  Nnu > 112 (but 120): the pivoted kernel (a 128 x 129 register tile spills, Gamma(w)
+// outgrows shared memory).
 template <int N, int T, int MINB>
 constexpr BseVariant padded_lu(const char* name) {
     return {&run_lu<N, T, 1, MINB, true, LDGA_LU_LOOKAHEAD, true>, name,
@@ -3053,15 +3049,12 @@ const BseVariant padded_lus[] = {padded_lu<8, 8, 8>("lu8p8"),     padded_lu<16, 
                                  padded_lu<80, 16, 1>("lu16p80"), padded_lu<96, 16, 1>("lu16p96"),
                                  padded_lu<112, 16, 1>("lu16p112")};
 const int padded_tiles[] = {8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 112};
-const BseVariant padded_iters[] = {{&run_group<48>, "iterg48", &run_group_pair<48>},
-                                   {&run_group<56>, "iterg56", &run_group_pair<56>},
-                                   {&run_group<64>, "iterg64", &run_group_pair<64>}};
 
-int padded_variant(int nnu, int prec, const BseVariant** out) {
+int padded_variant(int nnu, const BseVariant** out) {
     *out = nullptr;
     for (int i = 0; i < (int)(sizeof(padded_tiles) / sizeof(int)); ++i)
         if (nnu <= padded_tiles[i]) {
-            *out = prec == LDGA_PREC_MIXED && i >= 5 && i <= 7 ? &padded_iters[i - 5] : &padded_lus[i];
+            *out = &padded_lus[i];
             return 1;
         }
     return 0;
@@ -3079,7 +3072,7 @@ int variants_of(int nnu, int prec, const BseVariant** out) {
         case 120:
             if (prec == LDGA_PREC_MIXED) { *out = mixed_120; return (int)(sizeof(mixed_120) / sizeof(BseVariant)); }
             *out = fp64_120; return (int)(sizeof(fp64_120) / sizeof(BseVariant));
-        default: return padded_variant(nnu, prec, out);
+        default: return padded_variant(nnu, out);
     }
 #undef LDGA_BOX
 }

@@ -19,7 +19,7 @@
 // C is one Newton-Schulz step from the Jacobi seed, which is elementwise; only where its error bound
 // is above 1e-2 do the tensor-core iterations run.
 //
-// Built for tiles of 48, 56 and 64 rows (boxes of 42 .. 64), 8 warps of QW = 8 q: all of a CTA's 64 q share one
+// Built for tiles of 64 rows (the box of 60), 8 warps of QW = 8 q: all of a CTA's 64 q share one
 // inverse and one copy of Gamma, and 8 warps share an SM (k_bse_iter at N = 64 has 4).  The third-order
 // correction makes up for the wider groups: 4.9 passes per warp on the 2D 64^2 matrices, against
 // 5.6 at 32 q and second order.  Bound: the FP64 tensor path (three real products per complex tile, 16 cycles per
@@ -603,13 +603,9 @@ int launch_group(ldga_ctx* ctx, const BseArgs& a, const BseArgs* ad) {
 
 }  // namespace
 
-int run_bse_group(ldga_ctx* ctx, int tile, const BseArgs& a, const BseArgs* ad) {
+int run_bse_group(ldga_ctx* ctx, const BseArgs& a, const BseArgs* ad) {
+    constexpr int N = 64;
     if (!ctx->d_qperm) return ctx_fail(ctx, LDGA_ERR_ARG, "preconditioned BSE: q order buffer missing");
-    if (a.nnu > tile || a.nnu <= tile - 8) return ctx_fail(ctx, LDGA_ERR_ARG, "preconditioned BSE: tile and box size");
-    switch (tile) {
-        case 48: return launch_group<48, 8, 8, 1, 3>(ctx, a, ad);
-        case 56: return launch_group<56, 8, 8, 1, 3>(ctx, a, ad);
-        case 64: return launch_group<64, 8, 8, 1, 3>(ctx, a, ad);
-        default: return ctx_fail(ctx, LDGA_ERR_ARG, "preconditioned BSE: tile size");
-    }
+    if (a.nnu > N || a.nnu <= N - 8) return ctx_fail(ctx, LDGA_ERR_ARG, "preconditioned BSE: tile and box size");
+    return launch_group<N, 8, 8, 1, 3>(ctx, a, ad);
 }
