@@ -60,6 +60,8 @@ template <typename V>
 __device__ __forceinline__ V vmul(V a, V b) {
     V r; r.x = a.x * b.x - a.y * b.y; r.y = a.x * b.y + a.y * b.x; return r;
 }
+// a -= m * b, by the rounded product
+__device__ __forceinline__ void csubmul(double2& a, double2 m, double2 b) { a = csub(a, cmul(m, b)); }
 // a -= m * b
 template <typename V>
 __device__ __forceinline__ void vfnms(V& a, V m, V b) {
@@ -439,11 +441,21 @@ __global__ void __launch_bounds__(TR * TC * MPC, MINB) k_bse_tile(const BseArgs 
 // solution of later blocks: the row group folds its lanes' partial sums (three xor shuffles), the rhs
 // lane writes y_i = (z_i - sum) / b_ii, one named barrier, and every lane adds u_ij y_j of its column
 // of block r into the partial sums of the rows above.
-// The solution is verified by its FP64 backward error exactly like k_bse_tile (flag above 1e-12).
+// The solution is verified by its FP64 backward error exactly like k_bse_tile (flag above 1e-12; PAD: pad_tol).
 // PAD: a box of a.nnu < N rows on the tile of N: rows and columns beyond it are an identity block with a
 // zero right-hand side, so y stays 0 there.  Box sizes without kernels of their own run on the next tile;
 // they had the pivoted kernel (one matrix per CTA, three barriers and two divisions per step and element
 // loops with integer divisions) for every matrix: Nnu = 34, 84 q x 27 w 625 us per channel.
+// Their solutions keep the pivoted kernel's accuracy (errors of gamma within 6 %):
+//   - the updates subtract a rounded product (as there), not two fused products in turn, whose second
+//     rounding at the size of the element made every error sqrt(2) larger (y at Nnu = 34: 7.0e-16 with two
+//     FMAs, 5.7e-16 with the product, 5.1e-16 pivoted; 89 us a call either way, Nnu = 94 971 -> 1175 us);
+//   - gamma is formed by its quotient, as there;
+//   - a solution is accepted at the backward error a pivoted elimination has, not at 1e-12: pivoted, the
+//     largest seen are 2.6e-17 sqrt(Nnu) (5.3e-17 at 14, 1.2e-16 at 34, 2.5e-16 at 94), so twice that, and two
+//     roundings for the smallest boxes.  What is above (a small pivot: 13 of 315 matrices at Nnu = 14,
+//     errors to 1.6e-14) goes to the pivoted kernel.
+__device__ __forceinline__ double pad_tol(int n) { return fmax(2.2e-16, 5.5e-17 * sqrt((double)n)); }
 template <int N, int T>
 struct LuSmem {
     static constexpr int RT = (N + T - 1) / T;
@@ -560,7 +572,10 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a_m,
                 if (ra > (KC) || tr != ktc) {                                                    \
                     const double2 m = cb[tr + T * ra];                                           \
                     _Pragma("unroll") for (int c = (KC); c < CT; ++c) {                          \
-                        if ((COND) && (c > (KC) || tc > ktc)) vfnms<double2>(b[ra][c], m, u[c]); \
+                        if ((COND) && (c > (KC) || tc > ktc)) {                                  \
+                            if constexpr (PAD) csubmul(b[ra][c], m, u[c]);                       \
+                            else vfnms<double2>(b[ra][c], m, u[c]);                              \
+                        }                                                                        \
                     }                                                                            \
                 }                                                                                \
             }
@@ -711,19 +726,19 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a_m,
 
         // ---- chi and gamma = y / (chi0 (1 + s U chi))
         const double chi = st[3] / (a.beta * a.beta);
-        const bool ok = isfinite(chi) && isfinite(berr) && berr <= 1e-12;
+        const bool ok = isfinite(chi) && isfinite(berr) && berr <= (PAD ? pad_tol(nl) : 1e-12);
         if (t == 0) {
             a.chi[(size_t)q + (size_t)a.nq * w] = chi;
             a.flags[(size_t)q + (size_t)a.nq * w] = ok ? 0 : 1;
             if (!ok && a.fail_list) a.fail_list[atomicAdd(a.fail_count, 1)] = q + a.nq * w;
         }
-        const double rf = 1.0 / (1.0 + a.s * a.U * chi);
+        const double f = 1.0 + a.s * a.U * chi, rf = 1.0 / f;
 #pragma unroll
         for (int ra = 0; ra < RT; ++ra) {
             const int i = tr + T * ra;
             if (i < nl && tc == 0) {
                 const size_t ci = (size_t)q + (size_t)a.nq * (i + (size_t)nl * w);
-                a.gam[ci] = cscale(cmul(y[ra], dinv[i]), rf);
+                a.gam[ci] = PAD ? cdiv(y[ra], cscale(a.chi0[ci], f)) : cscale(cmul(y[ra], dinv[i]), rf);
             }
         }
         named_barrier(bar, G);   // shared buffers of this matrix are read before the next one writes
@@ -3034,7 +3049,7 @@ const BseVariant mixed_120[] = {{&run_jacobi<120, 32, 4, true>, "jac", &run_jaco
 
 // Box sizes without kernels of their own: the FP64 LU on the next tile up (padded), in every mode.  (MIXED on the
 // grouped iteration at 42..64 was no faster below 100 q and 50 to 4000 times further from the exact solution than
-// the FP64 elimination: 45 q x 25 w, Nnu = 46 202 us a call against 149, errors of chi 2.5e-14 to 4e-13
+// the FP64 elimination: 45 q x 25 w, Nnu = 46 202 us a call against 161, errors of chi 2.5e-14 to 4e-13
 // against 3e-16.)  Nnu > 112 (but 120): the pivoted kernel (a 128 x 129 register tile spills, Gamma(w)
 // outgrows shared memory).
 template <int N, int T, int MINB>
