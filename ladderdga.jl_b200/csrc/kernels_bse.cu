@@ -1390,6 +1390,13 @@ constexpr int kIterQ = 32;      // q per CTA: one preconditioner
 constexpr int kNsMaxIts = 6;    // Newton-Schulz iterations at most (tensor-core group inverse)
 constexpr float kNsTol = 1e-2f; // stop once (max row sum of |I - B_bar X|)^2 <= kNsTol
 constexpr double kIterTol = 1e-14;
+// A q iterates until its backward error is at most this, and is accepted at kIterTol.  At Nν = 30 the iteration
+// is the default in place of the FP32 elimination with FP64 refinement, which leaves most matrices at
+// 1e-16: stopped at 1e-14 its solutions were up to 10x further from the exact ones (2D 32^2, RPA-like vertex:
+// chi 1.8e-13 against 7e-14 and 1.7e-13 against 1.7e-14), at 1e-15 they are nearer (5.8e-15, 8.3e-15), in the
+// time of half a sweep more (113 us a call; 108).
+template <int NL>
+constexpr double kIterStop = NL == 30 ? 1e-15 : kIterTol;
 
 // TC: the FP32 product x += C r runs on tensor cores (mma.sync m16n8k8, TF32 operands, FP32
 // accumulation): C is kept as the A fragments of its real and imaginary parts, MT x KT tiles of
@@ -2212,7 +2219,7 @@ __global__ void __launch_bounds__(kIterQ * LPQ / QPL, MINB) k_bse_iter(const Bse
             }
             // normwise backward error |b - B x| / (|B| |x| + |b|), |b| = 1 for the forward solve
             if (!conv[c]) berr[c] = res / (rown[c] * xn + (ADJ ? bn[ADJ ? c : 0] : 1.0));
-            conv[c] = conv[c] || berr[c] <= kIterTol;
+            conv[c] = conv[c] || berr[c] <= kIterStop<NL>;
             all = all && conv[c];
         }
         passes = it + 1;
