@@ -674,8 +674,8 @@ int ldga_tune_save(const char* path) {
     for (int nnu = 1; nnu <= LDGA_MAX_NNU; ++nnu)
         for (int prec = LDGA_PREC_FP64_INV; prec <= LDGA_PREC_MIXED; ++prec) {
             const int n = bse_variant_count(nnu, prec);
-            const int i = bse_tuned_variant(nnu, prec);
-            if (n > 1 && i > 0 && i < n) std::fprintf(f, "bse %d %d %s\n", nnu, prec, bse_variant_name(nnu, prec, i));
+            const int i = bse_recorded_variant(nnu, prec);
+            if (n > 1 && i >= 0 && i < n) std::fprintf(f, "bse %d %d %s\n", nnu, prec, bse_variant_name(nnu, prec, i));
         }
     std::fclose(f);
     return LDGA_OK;
@@ -694,7 +694,7 @@ int ldga_bse_sweeps(ldga_ctx* ctx, int64_t* passes, int64_t* warps) {
 }
 
 const char* ldga_bse_config_name(int32_t nnu, int32_t precision, int32_t index) {
-    if (index < 0) index = bse_tuned_variant(nnu, precision);
+    if (index < 0) index = std::max(bse_recorded_variant(nnu, precision), 0);
     return bse_variant_name(nnu, precision, index);
 }
 

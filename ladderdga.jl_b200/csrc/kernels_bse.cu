@@ -3099,27 +3099,27 @@ int variants_of(int nnu, int prec, const BseVariant** out) {
 #undef LDGA_BOX
 }
 
-// chosen variant per (Nν, precision mode); absent = 0
+// recorded choices per (Nν, precision mode)
 std::mutex g_tune_mu;
 std::map<std::pair<int, int>, int> g_tune;
 
-int tuned_index(int nnu, int prec) {
+int recorded_variant(int nnu, int prec) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find({nnu, prec});
-    return it == g_tune.end() ? 0 : it->second;
+    return it == g_tune.end() ? -1 : it->second;
 }
 
-// The configuration a launch uses: the recorded choice, else entry 0, except that at Nν = 30 grids with many
-// q take the tensor-core iteration: 2D 32^2 (153 q, Nω = 31) 256 us for both channels against the warp LU's
-// 384, 3D 16^3 (165 q) 283 against 389.  With few q the groups' diagonals spread more and matrices are
-// left to the pivoted solve, so smaller grids keep the LU.
+// The configuration a launch uses: the recorded choice, else entry 0, except that at Nν = 30 grids of four or more
+// groups of 32 q (one inverse each) take the tensor-core iteration.  The elimination's time grows with the q, the
+// iteration's with the groups, and with few q a group's diagonals spread and cost sweeps.  Both channels, 31 ω,
+// random vertex / RPA-like vertex, elimination against iteration: 66 q 142 / 130 us against 212 / 111, 84 q 195 / 172
+// against 207 / 108, 91 q 196 / 174 against 191 / 105, 153 q 287 / 261 against 149 / 113, 165 q 310 / 268 against
+// 194 / 121, 325 q 547 / 484 against 190 / 151, 969 q 1497 / 1279 against 369 / 337.  (No grid has 92 .. 152 q.)
+// At Nν = 16 and 20 the random vertex breaks even at about 560 and 165 q; there the choice is left to the autotuner.
 int chosen_variant(const ldga_ctx* ctx) {
-    const int i = tuned_index(ctx->Nnu, ctx->prec);
-    if (i == 0 && ctx->Nnu == 30 && ctx->prec == LDGA_PREC_MIXED && ctx->Nq >= 150) {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        if (g_tune.find({30, LDGA_PREC_MIXED}) == g_tune.end()) return kIter30;
-    }
-    return i;
+    const int i = recorded_variant(ctx->Nnu, ctx->prec);
+    if (i >= 0) return i;
+    return ctx->Nnu == 30 && ctx->prec == LDGA_PREC_MIXED && (ctx->Nq + kIterQ - 1) / kIterQ >= 4 ? kIter30 : 0;
 }
 
 // The kernels see the ω shard as a whole problem of shard_nw frequencies: every array has ω as its
@@ -3259,7 +3259,13 @@ const char* bse_variant_name(int nnu, int prec, int i) {
     return (i >= 0 && i < n) ? v[i].name : nullptr;
 }
 
-int bse_tuned_variant(int nnu, int prec) { return tuned_index(nnu, prec); }
+int bse_recorded_variant(int nnu, int prec) { return recorded_variant(nnu, prec); }
+
+int bse_chosen_variant(const ldga_ctx* ctx) {
+    const BseVariant* v = nullptr;
+    const int nv = variants_of(ctx->Nnu, ctx->prec, &v), i = nv > 0 ? chosen_variant(ctx) : 0;
+    return i < nv ? i : 0;
+}
 
 void bse_set_variant(int nnu, int prec, int i) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -3289,8 +3295,7 @@ int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail) {
     const BseVariant* v = nullptr;
     const int nv = variants_of(ctx->Nnu, ctx->prec, &v);
     if (nv > 0) {
-        int i = chosen_variant(ctx);
-        if (i >= nv) i = 0;
+        const int i = bse_chosen_variant(ctx);
         LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count, 0, sizeof(int32_t), ctx->stream));
         a.fail_list = ctx->d_list;
         a.fail_count = ctx->d_count;
@@ -3319,8 +3324,7 @@ int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail) {
 int launch_bse_pair(ldga_ctx* ctx, int32_t* d_fail) {
     const BseVariant* v = nullptr;
     const int nv = variants_of(ctx->Nnu, ctx->prec, &v);
-    int i = nv > 0 ? chosen_variant(ctx) : 0;
-    if (i >= nv) i = 0;
+    const int i = bse_chosen_variant(ctx);
     if (nv == 0 || !v[i].run_pair) {
         const int st = launch_bse(ctx, LDGA_CH_M, d_fail);
         return st != LDGA_OK ? st : launch_bse(ctx, LDGA_CH_D, d_fail);

@@ -242,11 +242,12 @@ inline bool sharded(const ldga_ctx* c) { return c->w_lo != 0 || c->w_hi != c->Nw
 int require_unsharded(ldga_ctx* ctx, const char* what);
 
 bool bse_has_fast_path(int nnu);
-// BSE kernel configurations (autotuning): count and name per (Nν, precision), the chosen index,
-// and one launch of configuration i on the channel's current inputs.
+// BSE kernel configurations (autotuning): count and name per (Nν, precision), the recorded choice (-1: none),
+// the index a handle's launches use, and one launch of configuration i on the channel's current inputs.
 int bse_variant_count(int nnu, int prec);
 const char* bse_variant_name(int nnu, int prec, int i);
-int bse_tuned_variant(int nnu, int prec);
+int bse_recorded_variant(int nnu, int prec);
+int bse_chosen_variant(const ldga_ctx* ctx);
 void bse_set_variant(int nnu, int prec, int i);
 void bse_reset_variants();
 int bse_run_variant(ldga_ctx* ctx, int channel, int i);
