@@ -562,7 +562,7 @@ def tune(chain) -> str:
     else:
         for t in ("m", "d"):
             L.autotune_bse(chain.h, t, reps=3)
-    name = chain.lib.ldga_bse_config_name(ctx.Nnu, ctx.precision, -1)
+    name = chain.lib.ldga_bse_config(ctx.h)
     return name.decode() if name else "pivoted"
 
 
@@ -654,7 +654,7 @@ def roofline(stages: dict, chain, peaks: dict, sweeps=None, steps: int = 1) -> d
         # what the kernel executes: elimination of [B | 1] alone (BSE_EXEC_CMACS complex multiply-adds)
         exe = chans * nq * nw * 8.0 * BSE_EXEC_CMACS(nnu) / t / 1e12
         sm_mhz = peaks.get("sm_max_mhz", 1965.0)
-        cfg = chain.lib.ldga_bse_config_name(nnu, chain.ctx.precision, -1)
+        cfg = chain.lib.ldga_bse_config(chain.ctx.h)
         cfg = cfg.decode() if cfg else ""
         if cfg.startswith("iter"):
             # MIXED preconditioned solve: the FP64 residual passes set the bound.  Executed work from

@@ -228,8 +228,13 @@ int ldga_autotune_bse(ldga_ctx* ctx, int32_t channel, int32_t reps, int32_t* var
  * unknown names are ignored on load. */
 int ldga_tune_save(const char* path);
 int ldga_tune_load(const char* path);
-/* Name of BSE configuration `index` for (nnu, precision) -- index < 0: the one in use -- or NULL. */
+/* Name of BSE configuration `index` for (nnu, precision) -- index < 0: the recorded choice, else the
+ * default -- or NULL. */
 const char* ldga_bse_config_name(int32_t nnu, int32_t precision, int32_t index);
+/* Name of the BSE configuration this handle's launches use, or NULL (partial pivoting for every matrix).
+ * Without a recorded choice it can depend on the k-grid: at Nnu = 30 in MIXED, grids of more than 96
+ * irreducible q run the tensor-core iteration, smaller ones the default. */
+const char* ldga_bse_config(const ldga_ctx* ctx);
 /* Work counters of the MIXED preconditioned BSE since the last call (no reference counterpart:
  * diagnostics for rooflines): passes = residual evaluations summed over warps (each warp iterates
  * its q in lockstep), warps = warps that ran.  Both are reset by the call. */

@@ -29,7 +29,7 @@ EXPORTS = [
     "ldga_lambda_dm_evals", "ldga_set_stream", "ldga_profile", "ldga_stage_times", "ldga_launch_count",
     "ldga_get", "ldga_chain_m", "ldga_lambda0_noalloc", "ldga_batch_chain_m", "ldga_run_sc", "ldga_bse_vjp",
     "ldga_eom_vjp", "ldga_autotune_bse", "ldga_tune_save", "ldga_tune_load",
-    "ldga_tune_reset", "ldga_bse_config_name", "ldga_gloc_vjp", "ldga_epot_vjp", "ldga_chain_vjp",
+    "ldga_tune_reset", "ldga_bse_config_name", "ldga_bse_config", "ldga_gloc_vjp", "ldga_epot_vjp", "ldga_chain_vjp",
     "ldga_bse_sweeps", "ldga_profile_stages", "ldga_selftest_group_inverse", "ldga_set_omega_shard",
 ]
 GET_CHI0, GET_CHI, GET_GAMMA, GET_LAMBDA0, GET_SIGMA, GET_GLOC = 0, 1, 2, 3, 4, 5
@@ -131,6 +131,7 @@ def load(path: str | os.PathLike | None = None) -> C.CDLL:
         "ldga_tune_load": (C.c_int, [C.c_char_p]),
         "ldga_tune_reset": (C.c_int, []),
         "ldga_bse_config_name": (C.c_char_p, [I32, I32, I32]),
+        "ldga_bse_config": (C.c_char_p, [P]),
         "ldga_gloc_vjp": (C.c_int, [P, P, P, P, D, D, I32, I32, P, P]),
         "ldga_epot_vjp": (C.c_int, [P, I32, D, P, P]),
         "ldga_chain_vjp": (C.c_int, [P, P, D, D, I32, I32, P, P, I32, P, P, P]),

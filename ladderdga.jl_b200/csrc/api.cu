@@ -698,6 +698,10 @@ const char* ldga_bse_config_name(int32_t nnu, int32_t precision, int32_t index) 
     return bse_variant_name(nnu, precision, index);
 }
 
+const char* ldga_bse_config(const ldga_ctx* ctx) {
+    return ctx ? bse_variant_name(ctx->Nnu, ctx->prec, bse_chosen_variant(ctx)) : nullptr;
+}
+
 int ldga_tune_reset(void) {
     bse_reset_variants();
     return LDGA_OK;
