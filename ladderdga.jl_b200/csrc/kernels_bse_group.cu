@@ -8,9 +8,8 @@
 // until its FP64 backward error is small enough.
 //
 // What differs is the layout.  The products are formed transposed, X^T B^T and R^T C^T, with q on the
-// rows of the mma.sync tiles.  Lane (g, t) of a warp (g = lane / 4, t = lane % 4) owns, for q = g (and g + 8 with
-// QW = 16), the columns nu = 8 n + 2 t + e, e = 0, 1: exactly what the accumulator tiles give it (row g,
-// columns 2 t, 2 t + 1).  As an A operand a tile wants row g, column t: the k index is only summed over, so
+// rows of the mma.sync tiles.  Lane (g, t) of a warp (g = lane / 4, t = lane % 4) owns, for q = g, the columns
+// nu = 8 n + 2 t + e, e = 0, 1: exactly what the accumulator tiles give it (row g, columns 2 t, 2 t + 1).  As an A operand a tile wants row g, column t: the k index is only summed over, so
 // tile (n, e) takes nu = 8 n + 2 t + e as its column t, and the B operand is stored with the same
 // permutation.  x, r and the corrections therefore stay in registers in both roles, and a pass has
 // no shared-memory exchange and no warp synchronisation; in k_bse_iter each of its three products
@@ -19,7 +18,7 @@
 // C is one Newton-Schulz step from the Jacobi seed, which is elementwise; only where its error bound
 // is above 1e-2 do the tensor-core iterations run.
 //
-// Built for tiles of 64 rows (the box of 60), 8 warps of QW = 8 q: all of a CTA's 64 q share one
+// Built for tiles of 64 rows (the box of 60), 8 warps of 8 q: all of a CTA's 64 q share one
 // inverse and one copy of Gamma, and 8 warps share an SM (k_bse_iter at N = 64 has 4).  The third-order
 // correction makes up for the wider groups: 4.9 passes per warp on the 2D 64^2 matrices, against
 // 5.6 at 32 q and second order.  Bound: the FP64 tensor path (three real products per complex tile, 16 cycles per
@@ -39,7 +38,10 @@ constexpr int kGrpNsIts = 6;        // Newton-Schulz iterations at most
 constexpr float kGrpNsTol = 1e-2f;  // stop once (max row sum of |I - B_bar X|)^2 <= kGrpNsTol
 // Iterate to a backward error of 4e-15 (at most 10 sweeps for its sake), accept 1e-14 like k_bse_iter: stopping
 // at 1e-14 left the solutions of this contraction 2.2x further from the exact ones than k_bse_iter's, with
-// 4e-15 they are nearer (2.1e-15 against 3.7e-15, Nnu = 60, 2D 64^2) in the same time.
+// 4e-15 they are nearer (2.1e-15 against 3.7e-15, Nnu = 60, 2D 64^2) in the same time.  3e-15 and 2.5e-15 are nearer
+// still (1.3e-15, 0.8e-15); of these only 4e-15 passes test_config2_lambda_dm, whose Newton ends at a
+// root that depends on the last bits of chi: a change of this constant, or of an order of summation
+// before that Newton, can fail the test with every array at its parity tolerance.
 constexpr double kGrpStop = 4e-15, kGrpTol = 1e-14;
 constexpr int kGrpPatience = 10;
 
@@ -63,11 +65,11 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-// Shared memory of a CTA of NW warps with QW q each (QC = NW QW): [0, max(Gamma + C fragments, the
+// Shared memory of a CTA of NW warps with 8 q each (QC in all): [0, max(Gamma + C fragments, the
 // Newton-Schulz buffers)), then D, the row sums, the mean diagonal, reduction scratch.
-template <int N, int QW, int NW>
+template <int N, int NW>
 struct GrpSmem {
-    static constexpr int QC = QW * NW, NT = 32 * NW, T8 = N / 8;
+    static constexpr int QC = 8 * NW, NT = 32 * NW, T8 = N / 8;
     static constexpr int LDD = N + 1;                 // row stride of D: 16 bytes off a bank line per q
     static constexpr int LDE = N + 4;                 // row stride of dD (float2): 32 bytes off
     static constexpr int TPR = NT / N < 1 ? 1 : (NT / N > 4 ? 4 : NT / N);   // threads per row of the set-up
@@ -129,9 +131,9 @@ __device__ void gauss_jordan(float2* m, float2* col) {
 // C where one step from the Jacobi seed does not do: Newton-Schulz on the tensor cores (ns_inverse.cuh),
 // Gauss-Jordan where that does not converge either.  All threads; C fragments out, the Gamma fragments
 // (whose space the buffers take) written again from Gw.
-template <int N, int QW, int NW>
+template <int N, int NW>
 __device__ __forceinline__ void group_inverse(unsigned char* sm, const double2* __restrict__ Gw, int nl) {
-    using S = GrpSmem<N, QW, NW>;
+    using S = GrpSmem<N, NW>;
     using NSm = ns::NsSmem<N>;
     constexpr int NT = S::NT;
     const int tid = threadIdx.x;
@@ -201,11 +203,11 @@ __device__ __forceinline__ void group_inverse(unsigned char* sm, const double2* 
     __syncthreads();
 }
 
-template <int N, int QW, int NW, int MINB, int ORD>
-__global__ void __launch_bounds__(32 * NW, MINB) k_bse_group(const BseArgs a_m, const BseArgs a_d, int qpc,
+template <int N, int NW>
+__global__ void __launch_bounds__(32 * NW, 1) k_bse_group(const BseArgs a_m, const BseArgs a_d, int qpc,
                                                              const int32_t* __restrict__ perm) {
-    using S = GrpSmem<N, QW, NW>;
-    constexpr int NT = S::NT, T8 = S::T8, LDD = S::LDD, LDE = S::LDE, QC = S::QC, MT = QW / 8, TPR = S::TPR;
+    using S = GrpSmem<N, NW>;
+    constexpr int NT = S::NT, T8 = S::T8, LDD = S::LDD, LDE = S::LDE, QC = S::QC, TPR = S::TPR;
     extern __shared__ __align__(128) unsigned char gr_raw[];
     BseArgs a = a_m;
     if (blockIdx.z) {
@@ -357,38 +359,31 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_bse_group(const BseArgs a_m, 
         ek = (float)s.y;
         if (!(ek == ek)) ek = INFINITY;
     }
-    if (__syncthreads_or(!(ek * ek <= kGrpNsTol))) group_inverse<N, QW, NW>(gr_raw, Gw, nl);
+    if (__syncthreads_or(!(ek * ek <= kGrpNsTol))) group_inverse<N, NW>(gr_raw, Gw, nl);
     if (tid < 32) {
         tc05::fence_after();
         tc05::tmem_free(*slot, ns::NsSmem<N>::tmem_cols);
     }
 
-    // ---- this warp's q: QW consecutive ones of the group; no barrier from here on
-    const int ql0 = warp * QW;
+    // ---- this warp's q: 8 consecutive ones of the group; no barrier from here on
+    const int ql0 = warp * 8;
     if (ql0 >= nvalid) return;
-    const double2* Dl[MT];    // this lane's rows of D and dD (a q beyond QC has none: its last row)
-    const float2* El[MT];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-        const int qr = min(ql0 + 8 * mt + g, QC - 1);
-        Dl[mt] = Dq + qr * LDD;
-        El[mt] = Eq + qr * LDE;
-    }
+    const double2* Dl = Dq + (ql0 + g) * LDD;    // this lane's rows of D and dD
+    const float2* El = Eq + (ql0 + g) * LDE;
     const float4* Cl = reinterpret_cast<const float4*>(Cf) + lane;
     const double2* Gl = Gf + lane;
 
-    // w <- C w (TF32); w[mt][n][e] is element nu = 8 n + 2 t + e of q = g + 8 mt
-    auto apply = [&](float2 (&v)[MT][T8][2]) {
+    // v <- C v (TF32); v[n][e] is element nu = 8 n + 2 t + e of q = g; the tiles' rows 8..15 are zero
+    auto apply = [&](float2 (&v)[T8][2]) {
         uint32_t ar[T8][4], ai[T8][4];
 #pragma unroll
         for (int n = 0; n < T8; ++n)
 #pragma unroll
-            for (int e = 0; e < 2; ++e)
-#pragma unroll
-                for (int mt = 0; mt < 2; ++mt) {
-                    ar[n][mt + 2 * e] = mt < MT ? tf32(v[mt < MT ? mt : 0][n][e].x) : 0u;
-                    ai[n][mt + 2 * e] = mt < MT ? tf32(v[mt < MT ? mt : 0][n][e].y) : 0u;
-                }
+            for (int e = 0; e < 2; ++e) {
+                ar[n][2 * e] = tf32(v[n][e].x);
+                ai[n][2 * e] = tf32(v[n][e].y);
+                ar[n][2 * e + 1] = ai[n][2 * e + 1] = 0u;
+            }
 #pragma unroll
         for (int n = 0; n < T8; ++n) {
             float dre[4] = {0.f, 0.f, 0.f, 0.f}, dim[4] = {0.f, 0.f, 0.f, 0.f}, dni[4] = {0.f, 0.f, 0.f, 0.f},
@@ -404,190 +399,140 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_bse_group(const BseArgs a_m, 
                 mma_tf32(di2, ai[k], r0, r1);
             }
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    v[mt][n][e] = make_float2(dre[2 * mt + e] - dni[2 * mt + e], dim[2 * mt + e] + di2[2 * mt + e]);
+            for (int e = 0; e < 2; ++e) v[n][e] = make_float2(dre[e] - dni[e], dim[e] + di2[e]);
         }
     };
     // v <- (I - C dD + (C dD)^2) C v
-    auto correct = [&](float2 (&v)[MT][T8][2]) {
+    auto correct = [&](float2 (&v)[T8][2]) {
         apply(v);
-        float2 z[MT][T8][2];
+        float2 z[T8][2];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
+        for (int n = 0; n < T8; ++n)
 #pragma unroll
-            for (int n = 0; n < T8; ++n)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) z[mt][n][e] = v[mt][n][e];
+            for (int e = 0; e < 2; ++e) z[n][e] = v[n][e];
 #pragma unroll 1
-        for (int o = 0; o < ORD - 1; ++o) {      // rolled: unrolled, the compiler keeps dD of both orders and spills
+        for (int o = 0; o < 2; ++o) {      // rolled: unrolled, the compiler keeps dD of both orders and spills
 #pragma unroll
             for (int n = 0; n < T8; ++n)
 #pragma unroll
-                for (int e = 0; e < 2; ++e)
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt)
-                        z[mt][n][e] = fmul(El[mt][8 * n + 2 * t + e], z[mt][n][e]);
+                for (int e = 0; e < 2; ++e) z[n][e] = fmul(El[8 * n + 2 * t + e], z[n][e]);
             apply(z);
             const float sg = o ? 1.f : -1.f;
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
+            for (int n = 0; n < T8; ++n)
 #pragma unroll
-                for (int n = 0; n < T8; ++n)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        v[mt][n][e].x = fmaf(sg, z[mt][n][e].x, v[mt][n][e].x);
-                        v[mt][n][e].y = fmaf(sg, z[mt][n][e].y, v[mt][n][e].y);
-                    }
+                for (int e = 0; e < 2; ++e) {
+                    v[n][e].x = fmaf(sg, z[n][e].x, v[n][e].x);
+                    v[n][e].y = fmaf(sg, z[n][e].y, v[n][e].y);
+                }
         }
     };
 
-    double rown[MT], berr[MT];
-    bool conv[MT];
-    double2 x[MT][T8][2];
-    float2 rr[MT][T8][2];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-        rown[mt] = 0.0;
-        berr[mt] = 0.0;
-        conv[mt] = ql0 + 8 * mt + g >= nvalid;
-    }
+    double rown = 0.0, berr = 0.0;
+    bool conv = ql0 + g >= nvalid;
+    double2 x[T8][2];
+    float2 rr[T8][2];
 #pragma unroll
     for (int n = 0; n < T8; ++n)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int i = 8 * n + 2 * t + e;
-            const double2 gd = Gf[gfrag<N>(i, i)];
-            const double ra = rowabs[i];
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                const double2 d = Dl[mt][i];
-                rown[mt] = fmax(rown[mt], ra + fabs(gd.x + d.x) + fabs(gd.y + d.y));
-                rr[mt][n][e] = make_float2(i < nl ? 1.f : 0.f, 0.f);
-            }
+            const double2 gd = Gf[gfrag<N>(i, i)], d = Dl[i];
+            rown = fmax(rown, rowabs[i] + fabs(gd.x + d.x) + fabs(gd.y + d.y));
+            rr[n][e] = make_float2(i < nl ? 1.f : 0.f, 0.f);
         }
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-        rown[mt] = fmax(rown[mt], __shfl_xor_sync(0xffffffffu, rown[mt], 1));
-        rown[mt] = fmax(rown[mt], __shfl_xor_sync(0xffffffffu, rown[mt], 2));
-    }
+    rown = fmax(rown, __shfl_xor_sync(0xffffffffu, rown, 1));
+    rown = fmax(rown, __shfl_xor_sync(0xffffffffu, rown, 2));
     correct(rr);
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int n = 0; n < T8; ++n)
 #pragma unroll
-        for (int n = 0; n < T8; ++n)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) x[mt][n][e] = dmk((double)rr[mt][n][e].x, (double)rr[mt][n][e].y);
+        for (int e = 0; e < 2; ++e) x[n][e] = dmk((double)rr[n][e].x, (double)rr[n][e].y);
 
     int passes = 0;
     for (int it = 0;; ++it) {
         // r = 1 - (Gamma^T + D) x: three real tile products per complex tile (Karatsuba)
-        double res[MT], xn[MT];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) res[mt] = xn[mt] = 0.0;
+        double res = 0.0, xn = 0.0;
 #pragma unroll
         for (int n = 0; n < T8; ++n) {
-            double t1[MT][2], t2[MT][2], t3[MT][2];
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-                t1[mt][0] = t1[mt][1] = t2[mt][0] = t2[mt][1] = t3[mt][0] = t3[mt][1] = 0.0;
+            double t1[2] = {0.0, 0.0}, t2[2] = {0.0, 0.0}, t3[2] = {0.0, 0.0};
 #pragma unroll
             for (int k = 0; k < T8; ++k)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const double2 b = Gl[(n * 2 * T8 + 2 * k + e) * 32];
-                    const double bs = b.x + b.y;
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        const double2 xv = x[mt][k][e];
-                        mma_f64(t1[mt], xv.x, b.x);
-                        mma_f64(t2[mt], xv.y, b.y);
-                        mma_f64(t3[mt], xv.x + xv.y, bs);
-                    }
+                    const double2 b = Gl[(n * 2 * T8 + 2 * k + e) * 32], xv = x[k][e];
+                    mma_f64(t1, xv.x, b.x);
+                    mma_f64(t2, xv.y, b.y);
+                    mma_f64(t3, xv.x + xv.y, b.x + b.y);
                 }
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int i = 8 * n + 2 * t + e;
-                    const double2 xv = x[mt][n][e];
-                    const double2 dx = cmul(Dl[mt][i], xv);
-                    const double rx = (i < nl ? 1.0 : 0.0) - (t1[mt][e] - t2[mt][e] + dx.x);
-                    const double ry = -(t3[mt][e] - t1[mt][e] - t2[mt][e] + dx.y);
-                    res[mt] = fmax(res[mt], fabs(rx) + fabs(ry));
-                    xn[mt] = fmax(xn[mt], fabs(xv.x) + fabs(xv.y));
-                    rr[mt][n][e] = make_float2((float)rx, (float)ry);
-                }
-        }
-        bool all = true;
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-#pragma unroll
-            for (int o = 1; o < 4; o <<= 1) {
-                res[mt] = fmax(res[mt], __shfl_xor_sync(0xffffffffu, res[mt], o));
-                xn[mt] = fmax(xn[mt], __shfl_xor_sync(0xffffffffu, xn[mt], o));
-            }
-            if (!conv[mt]) berr[mt] = res[mt] / (rown[mt] * xn[mt] + 1.0);
-            conv[mt] = conv[mt] || berr[mt] <= (it < kGrpPatience ? kGrpStop : kGrpTol);
-            all = all && conv[mt];
-        }
-        passes = it + 1;
-        if (__all_sync(0xffffffffu, all) || it >= a.max_sweeps) break;
-        correct(rr);
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-            if (!conv[mt]) {
-#pragma unroll
-                for (int n = 0; n < T8; ++n)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        x[mt][n][e].x += (double)rr[mt][n][e].x;
-                        x[mt][n][e].y += (double)rr[mt][n][e].y;
-                    }
-            }
-    }
-    if (a.stats && lane == 0) {
-        atomicAdd(&a.stats[0], (unsigned long long)(passes * MT));
-        atomicAdd(&a.stats[1], (unsigned long long)MT);
-    }
-
-    // ---- chi, gamma = x / (chi0 (1 + s U chi)), flag (a q above the bound goes to the pivoted solve)
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-        double sx = 0.0;
-#pragma unroll
-        for (int n = 0; n < T8; ++n)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) sx += x[mt][n][e].x;      // padding rows of x are 0
-        sx += __shfl_xor_sync(0xffffffffu, sx, 1);
-        sx += __shfl_xor_sync(0xffffffffu, sx, 2);
-        const int ql = ql0 + 8 * mt + g;
-        if (ql >= nvalid) continue;
-        const int q = pw[ql];
-        const double chi = sx / (a.beta * a.beta);
-        const bool good = isfinite(chi) && isfinite(berr[mt]) && berr[mt] <= kGrpTol;
-        if (t == 0) {
-            a.chi[(size_t)q + (size_t)a.nq * w] = chi;
-            a.flags[(size_t)q + (size_t)a.nq * w] = good ? 0 : 1;
-            if (!good && a.fail_list) a.fail_list[atomicAdd(a.fail_count, 1)] = q + a.nq * w;
-        }
-        const double rf = 1.0 / (1.0 + a.s * a.U * chi);
-#pragma unroll
-        for (int n = 0; n < T8; ++n)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int i = 8 * n + 2 * t + e;
-                if (i < nl)
-                    a.gam[(size_t)q + (size_t)a.nq * (i + (size_t)nl * w)] = cscale(cmul(x[mt][n][e], Dl[mt][i]), rf);
+                const double2 xv = x[n][e], dx = cmul(Dl[i], xv);
+                const double rx = (i < nl ? 1.0 : 0.0) - (t1[e] - t2[e] + dx.x);
+                const double ry = -(t3[e] - t1[e] - t2[e] + dx.y);
+                res = fmax(res, fabs(rx) + fabs(ry));
+                xn = fmax(xn, fabs(xv.x) + fabs(xv.y));
+                rr[n][e] = make_float2((float)rx, (float)ry);
             }
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            res = fmax(res, __shfl_xor_sync(0xffffffffu, res, o));
+            xn = fmax(xn, __shfl_xor_sync(0xffffffffu, xn, o));
+        }
+        if (!conv) berr = res / (rown * xn + 1.0);
+        conv = conv || berr <= (it < kGrpPatience ? kGrpStop : kGrpTol);
+        passes = it + 1;
+        if (__all_sync(0xffffffffu, conv) || it >= a.max_sweeps) break;
+        correct(rr);
+        if (!conv) {
+#pragma unroll
+            for (int n = 0; n < T8; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    x[n][e].x += (double)rr[n][e].x;
+                    x[n][e].y += (double)rr[n][e].y;
+                }
+        }
     }
+    if (a.stats && lane == 0) {
+        atomicAdd(&a.stats[0], (unsigned long long)passes);
+        atomicAdd(&a.stats[1], 1ull);
+    }
+
+    // ---- chi, gamma = x / (chi0 (1 + s U chi)), flag (a q above the bound goes to the pivoted solve)
+    double sx = 0.0;
+#pragma unroll
+    for (int n = 0; n < T8; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) sx += x[n][e].x;      // padding rows of x are 0
+    sx += __shfl_xor_sync(0xffffffffu, sx, 1);
+    sx += __shfl_xor_sync(0xffffffffu, sx, 2);
+    const int ql = ql0 + g;
+    if (ql >= nvalid) return;
+    const int q = pw[ql];
+    const double chi = sx / (a.beta * a.beta);
+    const bool good = isfinite(chi) && isfinite(berr) && berr <= kGrpTol;
+    if (t == 0) {
+        a.chi[(size_t)q + (size_t)a.nq * w] = chi;
+        a.flags[(size_t)q + (size_t)a.nq * w] = good ? 0 : 1;
+        if (!good && a.fail_list) a.fail_list[atomicAdd(a.fail_count, 1)] = q + a.nq * w;
+    }
+    const double rf = 1.0 / (1.0 + a.s * a.U * chi);
+#pragma unroll
+    for (int n = 0; n < T8; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int i = 8 * n + 2 * t + e;
+            if (i < nl) a.gam[(size_t)q + (size_t)a.nq * (i + (size_t)nl * w)] = cscale(cmul(x[n][e], Dl[i]), rf);
+        }
 }
 
-template <int N, int QW, int NW, int MINB, int ORD>
+template <int N, int NW>
 int launch_group(ldga_ctx* ctx, const BseArgs& a, const BseArgs* ad) {
-    using S = GrpSmem<N, QW, NW>;
-    auto kern = k_bse_group<N, QW, NW, MINB, ORD>;
+    using S = GrpSmem<N, NW>;
+    auto kern = k_bse_group<N, NW>;
     LDGA_CUDA(ctx, set_smem(ctx, kern, S::bytes));
     StageTimer st_(ctx, LDGA_STAGE_BSE);
     const int qo = bse_ensure_qorder(ctx, a, a.nnu);
@@ -616,5 +561,5 @@ int run_bse_group(ldga_ctx* ctx, const BseArgs& a, const BseArgs* ad) {
     constexpr int N = 64;
     if (!ctx->d_qperm) return ctx_fail(ctx, LDGA_ERR_ARG, "preconditioned BSE: q order buffer missing");
     if (a.nnu > N || a.nnu <= N - 8) return ctx_fail(ctx, LDGA_ERR_ARG, "preconditioned BSE: tile and box size");
-    return launch_group<N, 8, 8, 1, 3>(ctx, a, ad);
+    return launch_group<N, 8>(ctx, a, ad);
 }

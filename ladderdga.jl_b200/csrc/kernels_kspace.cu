@@ -49,7 +49,10 @@ __global__ void __launch_bounds__((kThr<DIM, N, TC>), (kMinB<DIM, N, TC>)) k_glo
 //   chi0(q, nu'', w) = conj(chi0(q, nu, w)),  nu'' = -nu - w - 1,
 // and a pair whose partner lies in the box is computed once: `pairs` lists the representatives
 // (pair index vi + Nnu wi, partner's index or -1), built on the host with the handle.
-// The scale goes onto the product before the transform (one multiplication per input either way).
+// The scale goes onto the product before the transform (one multiplication per input either way, equally accurate:
+// 4e-16).  Which of two such roundings is taken decides where the lambda_m Newton of the 3D 32^3 test input, which
+// steps into a region of poles, ends: after the transform, tests of that root and of lambda_dm fail
+// with every array at its parity tolerance.
 // Measured, cold caches: 3D 32^3, Nnu = 40, Nw = 41 (1040 vectors) 35 us, 72 us with the unfolded
 // matrix at two threads per column; 2D 64^2, Nnu = 60, Nw = 61 (2310 vectors) 25 us, 108 us before.
 // ---------------------------------------------------------------------------------------------

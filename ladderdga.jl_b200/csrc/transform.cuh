@@ -163,7 +163,8 @@ struct TransformPlan {
         return best;
     }
     static constexpr int NP = pick();
-    // threads: an item of stages x each, and at most 3 (3D) or 4 (2D) wedge points of the loads and stores
+    // threads: an item of stage x each; more, up to 352, where that brings the wedge points of a thread's loads and
+    // stores down to 3 (3D) or 4 (2D) (2D 64^2 would need 576 and keeps 288 threads with 8 points)
     static constexpr int LDQ = DIM == 3 ? 3 : 4;
     static constexpr int NT_I = (NP * 2 * COLS + 31) / 32 * 32, NT_L = ((NP * S::NQ + LDQ - 1) / LDQ + 31) / 32 * 32;
     static constexpr int NT = NT_L > NT_I && NT_L <= 352 ? NT_L : NT_I;
