@@ -118,7 +118,7 @@ __global__ void __launch_bounds__((kThrOne<DIM, N, TC>), 1) k_eom_inverse(
 // SMs' slots times the steps of one CTA (3D 32^3, 20 ν x 41 ω: 2 ω per CTA in 1.4 rounds 48 us, 3 ω
 // in one round 41 us; 2D 64^2, 22 ν x 61 ω: 2 ω 36 us, 5 ω 30 us).
 // The split is not monotone in numax: fewer ν can need more partial sums (2D 64^2, 61 ω: 270 rows at
-// 30 ν, 589 at 19), so the handle's buffer is sized for every numax at once (eom_partial_need).
+// 30 ν, 589 at 19), so the handle's buffer is sized for every numax up to n_iv at once (eom_partial_need).
 template <int DIM, int N>
 EomShape eom_shape(int numax, int nw, bool tc) {
     using P = TransformPlan<DIM, N>;
@@ -152,7 +152,7 @@ EomShape eom_shape_of(ldga_ctx* ctx, int numax, int nw) {
 template <int DIM, int N>
 size_t partial_need(ldga_ctx* ctx) {
     size_t need = 0;
-    for (int numax = 1; numax <= ctx->Nnu; ++numax) {
+    for (int numax = 1; numax <= ctx->sp.n_iv; ++numax) {
         const int wpc = eom_shape_of<DIM, N>(ctx, numax, ctx->Nw).wpc;
         need = std::max(need, (size_t)((ctx->Nw + wpc - 1) / wpc) * numax * ctx->Nq);
     }
@@ -166,7 +166,7 @@ int run_eom(ldga_ctx* ctx, int numax, double lam_m, double lam_d, const double* 
     const EomShape shape = eom_shape_of<DIM, N>(ctx, numax, nws);
     const int wpc = shape.wpc, np = shape.np;
     const int nchunk = (nws + wpc - 1) / wpc;
-    // allocated with the handle; only an ω shard can need more
+    // allocated with the handle; numax above n_iv and an ω shard can need more
     const int gs = grow_buffer(ctx, &ctx->d_partial, &ctx->partial_elems, (size_t)nchunk * numax * ctx->Nq);
     if (gs != LDGA_OK) return gs;
     EomArgs a;

@@ -297,7 +297,7 @@ int launch_lambda0(ldga_ctx* ctx);
 int launch_lambda0_vjp(ldga_ctx* ctx, const double2* l0_bar, double2* chi0_bar);
 // dE_pot,1/dΣ_ladder [Nq, numax] with μ following the filling condition (calc_E after G_from_Σladder!)
 int launch_epot_vjp(ldga_ctx* ctx, int numax, double mu, const double2* sigma, double2* out);
-// Elements of the EoM's partial sums that hold every numax of the handle's box at the whole ω range
+// Elements of the EoM's partial sums that hold every numax up to n_iv at the whole ω range
 size_t eom_partial_need(ldga_ctx* ctx);
 // EoM forward + inverse.  lam_*_dev (may be null) are device scalars added to lam_m / lam_d.
 int launch_eom(ldga_ctx* ctx, int numax, double lam_m, double lam_d, const double* lam_m_dev,

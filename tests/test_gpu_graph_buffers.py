@@ -58,7 +58,7 @@ def test_replay_after_other_numbers_of_nu(dim, ns, n_iv, n_iw, require_gpu):
     assert same(run(1), want)                 # captures
     assert same(run(1), want)                 # replays
     ctx = h.ctx
-    for numax in range(1, n_iv + 1):
+    for numax in range(1, 2 * n_iv + 1):
         ctx.call("ldga_eom", 0.5, 0.0, numax, 1, h.χloc_m_sum, None)
     assert same(run(1), want)
     lm, ld = C.c_double(), C.c_double()
