@@ -36,14 +36,14 @@ namespace {
 
 constexpr int kGrpNsIts = 6;        // Newton-Schulz iterations at most
 constexpr float kGrpNsTol = 1e-2f;  // stop once (max row sum of |I - B_bar X|)^2 <= kGrpNsTol
-// Iterate to a backward error of 4e-15 (at most 10 sweeps for its sake), accept 1e-14 like k_bse_iter: stopping
+// Iterate to a backward error of 4e-15, accept 1e-14 like k_bse_iter (a matrix that has not got below 4e-15 at the
+// sweep limit): stopping
 // at 1e-14 left the solutions of this contraction 2.2x further from the exact ones than k_bse_iter's, with
 // 4e-15 they are nearer (2.1e-15 against 3.7e-15, Nnu = 60, 2D 64^2) in the same time.  3e-15 and 2.5e-15 are nearer
 // still (1.3e-15, 0.8e-15); of these only 4e-15 passes test_config2_lambda_dm, whose Newton ends at a
 // root that depends on the last bits of chi: a change of this constant, or of an order of summation
 // before that Newton, can fail the test with every array at its parity tolerance.
 constexpr double kGrpStop = 4e-15, kGrpTol = 1e-14;
-constexpr int kGrpPatience = 10;
 
 __device__ __forceinline__ double2 dmk(double r, double i) { return make_double2(r, i); }
 __device__ __forceinline__ uint32_t tf32(float x) {
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_bse_group(const BseArgs a_m, con
             xn = fmax(xn, __shfl_xor_sync(0xffffffffu, xn, o));
         }
         if (!conv) berr = res / (rown * xn + 1.0);
-        conv = conv || berr <= (it < kGrpPatience ? kGrpStop : kGrpTol);
+        conv = conv || berr <= kGrpStop;
         passes = it + 1;
         if (__all_sync(0xffffffffu, conv) || it >= a.max_sweeps) break;
         correct(rr);
