@@ -165,7 +165,7 @@ int alloc_all(ldga_ctx* c) {
     TRY(dev_alloc(c, &c->d_red, 64 + 2 * nnu * nw + 64 + 3 * kDmSlot));
     TRY(dev_alloc(c, &c->d_flags, nq * nw));
     TRY(dev_alloc(c, &c->d_list, nq * nw));
-    TRY(dev_alloc(c, &c->d_count, 4));
+    TRY(dev_alloc(c, &c->d_count, 8));
     TRY(dev_alloc(c, &c->d_qperm, nq * nw));
     TRY(dev_alloc(c, &c->d_iter_stats, 2));
     TRY(grow_buffer(c, &c->d_partial, &c->partial_elems, eom_partial_need(c)));
@@ -591,7 +591,7 @@ int ldga_bse_vjp(ldga_ctx* ctx, int32_t channel, const double* chi_bar, const do
     TRY(sc.get(ctx, &d_y, qvw));
     TRY(sc.get(ctx, &d_z, qvw));
     TRY(sc.get(ctx, &d_Gb, vvw));
-    LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count, 0, 2 * sizeof(int32_t), ctx->stream));
+    LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count, 0, 8 * sizeof(int32_t), ctx->stream));
     TRY(launch_bse_adj(ctx, channel, d_xb, d_gb, d_c0b, d_y, d_z, d_Gb, ctx->d_count + 1));
     int32_t cnt[2] = {0, 0};
     TRY(copy(ctx, cnt, ctx->d_count, 2 * sizeof(int32_t)));
@@ -1004,7 +1004,7 @@ int ldga_chain_vjp(ldga_ctx* ctx, const double* sigma_bar, double lam_m, double 
     TRY(sc.get(ctx, &d_z, qvw));
     TRY(sc.get(ctx, &d_Gm, vvw));
     TRY(sc.get(ctx, &d_Gd, vvw));
-    LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count, 0, 2 * sizeof(int32_t), ctx->stream));
+    LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count, 0, 8 * sizeof(int32_t), ctx->stream));
     TRY(launch_bse_adj(ctx, LDGA_CH_M, d_xm, d_gm, d_c0b, d_y, d_z, d_Gm, ctx->d_count + 1, false));
     TRY(launch_bse_adj(ctx, LDGA_CH_D, d_xd, d_gd, d_c0b, d_y, d_z, d_Gd, ctx->d_count + 1, true));
     TRY(launch_lambda0_vjp(ctx, d_l0, d_c0b));

@@ -3371,8 +3371,8 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
     if (!ctx->d_list2)
         LDGA_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->d_list2), (size_t)ctx->Nq * ctx->Nw * sizeof(int32_t)));
     a.fail_list = ctx->d_list2;
-    a.fail_count = ctx->d_count + 3;
-    LDGA_CUDA(ctx, cudaMemsetAsync(ctx->d_count + 2, 0, 2 * sizeof(int32_t), ctx->stream));   // both lists
+    int32_t* counts = ctx->d_count + 4 + 2 * (channel == LDGA_CH_D);   // left by the iteration, by the LU
+    a.fail_count = counts + 1;
     int st = LDGA_OK;
     if (ctx->prec == LDGA_PREC_MIXED && ctx->Nnu == 40) {
         // MIXED: the preconditioned iteration on the transposed systems, the LU for what it leaves
@@ -3393,7 +3393,7 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
         b.chi = nullptr;
         b.stats = nullptr;
         b.fail_list = ctx->d_list;
-        b.fail_count = ctx->d_count + 2;
+        b.fail_count = counts;
         st = run_iter_impl<N, 8, 2, 2, true, true, true, true, true, N, true>(ctx, b, nullptr);
         if (st != LDGA_OK) return st;
         // chi0_bar of the solved matrices first: the LU below clears the flags of those it solves
@@ -3401,7 +3401,7 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
         LDGA_LAUNCHED(ctx, "k_adj_chi0bar");
         BseAdjArgs al = a;
         al.list = ctx->d_list;
-        al.count = ctx->d_count + 2;
+        al.count = counts;
         const size_t sm = (size_t)N * N * sizeof(double2) + LuSmem<N, 8>::bytes + 2 * N * sizeof(double2) + 16;
         auto kern = k_bse_adj<N, 8, 6>;
         LDGA_CUDA(ctx, set_smem(ctx, kern, sm));
@@ -3425,7 +3425,7 @@ int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const doub
     }
     if (st != LDGA_OK) return st;
     a.list = ctx->d_list2;
-    a.count = ctx->d_count + 3;
+    a.count = counts + 1;
     const size_t smp = bse_pivot_smem(ctx->Nnu);      // at most 60 rows: 60 KB
     LDGA_CUDA(ctx, set_smem(ctx, k_bse_adj_pivot, smp));
     k_bse_adj_pivot<<<LDGA_PIVOT_GRID, 256, smp, ctx->stream>>>(a, d_fail);

@@ -112,6 +112,8 @@ struct ldga_ctx {
     int32_t* d_list = nullptr;     // matrices left to the pivoted solve (the m channel's list of a pair launch)
     int32_t* d_list2 = nullptr;    // the d channel's list of a pair launch
     double2* d_gamma_t = nullptr;  // MIXED BSE adjoint: Gamma(w) transposed [Nnu, Nnu, Nw]
+    // [0] list of one channel's solve, [1] matrices left unsolved, [2..3] lists of a pair launch,
+    // [4 + 2 channel ..] lists of a channel's adjoint (iteration, LU)
     int32_t* d_count = nullptr;
     double2* d_pivot_scratch = nullptr;   // pivoted fallback matrices in HBM when N (N+1) does not fit shared memory
     int2* d_bub_pairs = nullptr;          // bubble pairs computed directly (pair, conjugate partner or -1)
@@ -274,7 +276,7 @@ int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail);
 int launch_bse_pair(ldga_ctx* ctx, int32_t* d_fail);
 // Adjoint of one BSE channel: chi0_bar (written, or added to when accumulate), y and z buffers
 // [Nq, Nnu, Nw], Gamma_bar [Nnu, Nnu, Nw]; the number of adjoint solves that stay non-finite with partial
-// pivoting is added to d_fail.
+// pivoting is added to d_fail.  The caller zeroes d_count (all 8) before the first channel.
 int launch_bse_adj(ldga_ctx* ctx, int channel, const double* chi_bar, const double2* gam_bar, double2* chi0_bar,
                    double2* ybuf, double2* zbuf, double2* gamma_bar, int32_t* d_fail, bool accumulate = false);
 // Adjoint of the EoM at (lam_m, lam_d): sbar [numax][Nq] -> gm_bar, gd_bar, l0_bar [Nq, Nnu, Nw] (pre-zeroed;
