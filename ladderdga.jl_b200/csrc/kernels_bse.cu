@@ -652,7 +652,10 @@ __global__ void __launch_bounds__(T * T * MPC, MINB) k_bse_lu(const BseArgs a_m,
                             const double2 m = cb[tr + T * ra];
     #pragma unroll
                             for (int c = kc; c < CT; ++c) {
-                                if (c > kc || tc > ktc) vfnms<double2>(b[ra][c], m, u[c]);
+                                if (c > kc || tc > ktc) {
+                                    if constexpr (PAD) csubmul(b[ra][c], m, u[c]);
+                                    else vfnms<double2>(b[ra][c], m, u[c]);
+                                }
                             }
                         }
                     }
@@ -3287,7 +3290,7 @@ int bse_run_variant(ldga_ctx* ctx, int channel, int i) {
 // One channel: the configuration appends the matrices it leaves above its backward-error bound to d_list (count
 // in d_count[0]), a grid-stride pivoted launch re-solves the list (zero work when it is empty) and counts
 // into *d_fail what stays non-finite.  Appending takes the place of two passes over the flags around the
-// pivoted launch: a call at Nnu = 40 on 32^3 takes 590 us, 610 us with them, at Nnu = 34 on 12^3 in FP64
+// pivoted launch: a call at Nnu = 40 on 32^3 took 590 us, 610 us with them, at Nnu = 34 on 12^3 in FP64
 // 271 us (290 us).
 int launch_bse(ldga_ctx* ctx, int channel, int32_t* d_fail) {
     BseArgs a = bse_args(ctx, channel);
