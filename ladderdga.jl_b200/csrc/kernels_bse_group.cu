@@ -539,17 +539,18 @@ int launch_group(ldga_ctx* ctx, const BseArgs& a, const BseArgs* ad) {
     if (qo != LDGA_OK) return qo;
     // As few groups as QC allows, of about the same number of q each: more and smaller groups took more rounds
     // on the SMs at the same time per CTA (2D 64^2, Nnu = 60: 64 q per CTA 497 us, 47 q 551 us).  Groups of 32 where
-    // one channel's have an SM each and both channels' take no more rounds than groups of 64: with four warps,
-    // one per sub-partition, a CTA has 0.77 of the time of eight, and narrower groups need fewer sweeps.  One
-    // channel, random / RPA-like vertex, groups of 64 against 32: 153 q x 7 w 231 / 150 us against 126 / 116, 231 q x 7 w
-    // 188 / 151 against 127 / 116, 91 q x 17 w 286 / 156 against 194 / 115; where both channels' take a round more,
-    // that launch loses (153 q x 17 w, RPA-like, 173 us against 201).  The line is the same for one channel, for
-    // both and for a shard of the w, so a matrix has the same group, and bits, in each.
+    // one channel's have an SM each and the launch takes no more rounds than with groups of 64: with four
+    // warps, one per sub-partition, a CTA has 0.77 of the time of eight, and narrower groups need fewer sweeps.  One
+    // channel, random / RPA-like vertex, groups of 64 against 32: 153 q x 7 w 231 / 150 us against 126 / 116, 153 q x 17 w
+    // 228 / 147 against 126 / 115, 91 q x 17 w 286 / 156 against 194 / 115; a round more loses (both channels, 153 q x
+    // 17 w, RPA-like, 173 us against 201; one channel, 325 q x 17 w, 164 / 151 against 172 / 188).  The line depends on the whole
+    // range of w, so a matrix has the same group, and bits, in a shard; one channel and both may differ by it.
+    const int z = ad ? 2 : 1;
     auto rounds = [](long ctas) { return (ctas + 147) / 148; };
     const long c32 = (long)((a.nq + 31) / 32) * ctx->Nw, c64 = (long)((a.nq + 63) / 64) * ctx->Nw;
-    const int per = c32 <= 148 && rounds(2 * c32) <= rounds(2 * c64) ? 32 : S::QC;
+    const int per = c32 <= 148 && rounds(z * c32) <= rounds(z * c64) ? 32 : S::QC;
     const int nct = (a.nq + per - 1) / per, qpc = (a.nq + nct - 1) / nct;
-    dim3 grid((a.nq + qpc - 1) / qpc, a.nw, ad ? 2 : 1);
+    dim3 grid((a.nq + qpc - 1) / qpc, a.nw, z);
     kern<<<grid, S::NT, S::bytes, ctx->stream>>>(a, ad ? *ad : a, qpc, ctx->d_qperm);
     LDGA_LAUNCHED(ctx, "k_bse_group");
     return LDGA_OK;
